@@ -201,12 +201,14 @@ size_t trtri_scratch_elems(int64_t m, int64_t batch) { return (size_t)trtri_chun
 // Batched L^{-1} in chunks of kTrtriChunk blocks: SIMT products natively,
 // tensor-core products in mixed mode.
 template <typename T>
-cudaError_t trtri_run(const Ctx& cx, const T* L, int64_t m, int64_t batch, T* Linv, T* scratch, cudaStream_t s) {
+cudaError_t trtri_run(const Ctx& cx, const T* L, int64_t m, int64_t batch, T* Linv, T* scratch, cudaStream_t s,
+                      int64_t sub = 0) {
     const int64_t mm = m * m;
     for (int64_t j0 = 0; j0 < batch; j0 += kTrtriChunk) {
         const int64_t nb = (batch - j0) < kTrtriChunk ? (batch - j0) : kTrtriChunk;
         cudaError_t e = cx.slices == 0
-                            ? trtri_batched<T>(L + j0 * mm, m, mm, m, nb, Linv + j0 * mm, m, mm, scratch, s)
+                            ? trtri_batched<T>(L + j0 * mm, m, mm, m, nb, Linv + j0 * mm, m, mm, scratch, s,
+                                               nullptr, nullptr, sub)
                             : trtri_batched<T>(L + j0 * mm, m, mm, m, nb, Linv + j0 * mm, m, mm, scratch, s,
                                                ctx_gemm<T>, (void*)&cx);
         if (e != cudaSuccess) return e;
@@ -1010,14 +1012,24 @@ int pobtas_native(const sgb_bta* m, T* Bm, int64_t nrhs, int64_t ldb, char trans
 
     if (nrhs == 0) return SGB_OK;
     Ctx native;
-    // have_linv: the workspace holds the inverses from an earlier call with this factor
+    // the whole sweep as one launch, which needs the inverses of the diagonal
+    // sub-blocks only; the products below take the solves that leave the last
+    // block to the caller, very many columns and very wide blocks
+    const bool chain = !partial && solve_chain_ok<T>(m, nrhs, s);
+    const int64_t sub = chain ? solve_sub() : 0;
+    // have_linv: the workspace holds the inverses from an earlier call with
+    // this factor and the same number of columns
     if (!have_linv) {
         // with xall the block inverses exist already, as L_ii^{-T} (read transposed)
-        if (!xall) SGB_TRY(trtri_run<T>(native, D, b, n, Linv, trs, s));
-        if (a && !partial) SGB_TRY(trtri_run<T>(native, Tp, a, 1, Ltinv, trs, s));
+        if (!xall) SGB_TRY(trtri_run<T>(native, D, b, n, Linv, trs, s, sub));
+        if (a && !partial) SGB_TRY(trtri_run<T>(native, Tp, a, 1, Ltinv, trs, s, sub));
     }
     const T* Li = xall ? xall : Linv;
     const int tl = xall ? 1 : 0;
+    if (chain) {
+        SGB_TRY(solve_chain<T>(m, Bm, nrhs, ldb, trans != 'N', Li, xall != nullptr, Ltinv, s));
+        return SGB_OK;
+    }
 
     if (trans == 'N') {
         const int64_t last = partial ? n - 1 : n;
@@ -1551,7 +1563,7 @@ int plan_item(const sgb_bta* m, int ops, int precision, void* rhs, int64_t nrhs,
         sgb_pobtas_workspace_size(m, nrhs, precision, &need);
         if ((rc = check_ws(w, wb, need))) return rc;
         rc = pobtas_native<double>(m, (double*)rhs, nrhs, nrhs, 'N', 0, w, s, false, xa);
-        if (rc == SGB_OK) rc = pobtas_native<double>(m, (double*)rhs, nrhs, nrhs, 'T', 0, w, s, false, xa);
+        if (rc == SGB_OK) rc = pobtas_native<double>(m, (double*)rhs, nrhs, nrhs, 'T', 0, w, s, true, xa);
         if (rc) return rc;
     }
     if (ops & SGB_OP_POBTASI) {

@@ -137,11 +137,24 @@ bool capture_tc_split();
 // Full triangular inverse of `batch` lower-triangular m x m blocks:
 // Linv_j = L_j^{-1} (zeros above the diagonal).  Scratch: batch*m*m T.
 // The row-sweep products go through `fn(fnctx, ...)` when given, else the
-// SIMT kernel.
+// SIMT kernel.  With `sub` > 0 (a power of two times kTile) only the inverses
+// of the diagonal sub-blocks of `sub` rows are formed, in place of the whole.
 template <typename T>
 cudaError_t trtri_batched(const T* L, int64_t ldl, int64_t strideL, int64_t m, int64_t batch,
                           T* Linv, int64_t ldx, int64_t strideX, T* scratch, cudaStream_t s,
-                          GemmFn<T> fn = nullptr, void* fnctx = nullptr);
+                          GemmFn<T> fn = nullptr, void* fnctx = nullptr, int64_t sub = 0);
+
+// Whole-sweep triangular solve in one cluster launch (sgb_solve.cu).  `Li`
+// (n, b, b) holds the inverses of the diagonal sub-blocks of solve_sub() rows
+// of every L_ii at their places (their transposes with li_trans), `Lti` (a, a)
+// the same of the tip.  solve_chain_ok: whether the sizes fit it (otherwise
+// solve_chain returns cudaErrorNotSupported).
+int solve_sub();
+template <typename T>
+bool solve_chain_ok(const sgb_bta* m, int64_t nrhs, cudaStream_t s);
+template <typename T>
+cudaError_t solve_chain(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, const T* Li, bool li_trans,
+                        const T* Lti, cudaStream_t s);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

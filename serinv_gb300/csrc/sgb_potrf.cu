@@ -165,12 +165,16 @@ cudaError_t factor_column_block(T* diag, int64_t m, int64_t ldd, RowSet<T> r1, R
 
 template <typename T>
 cudaError_t trtri_batched(const T* L, int64_t ldl, int64_t strideL, int64_t m, int64_t batch, T* Linv,
-                          int64_t ldx, int64_t strideX, T* scratch, cudaStream_t s, GemmFn<T> fn, void* fnctx) {
+                          int64_t ldx, int64_t strideX, T* scratch, cudaStream_t s, GemmFn<T> fn, void* fnctx,
+                          int64_t sub) {
     auto gemm = [&](GemmProb<T>* p, int np) { return fn ? fn(fnctx, p, np, s) : gemm_simt<T>(p, np, s); };
     if (m <= 0 || batch <= 0) return cudaSuccess;
     cudaError_t err;
-    // Zero everything first: the recursion writes only the lower blocks.
-    if (ldx == m && strideX == m * m) {
+    // Zero everything first: the recursion writes only the lower blocks (a
+    // single tile is written whole).
+    if (m <= kTile) {
+        err = cudaSuccess;
+    } else if (ldx == m && strideX == m * m) {
         err = cudaMemsetAsync(Linv, 0, (size_t)(batch * m * m) * sizeof(T), s);
     } else {
         err = cudaMemset2DAsync(Linv, (size_t)ldx * sizeof(T), 0, (size_t)m * sizeof(T),
@@ -185,7 +189,7 @@ cudaError_t trtri_batched(const T* L, int64_t ldl, int64_t strideL, int64_t m, i
     // four to a grouped launch; every problem is batched over the blocks.
     // Scratch per block: the products L21 X11 of one level (<= m*m/2 + h*h).
     const int64_t sstride = m * m;
-    for (int64_t h = kTile; h < m; h *= 2) {
+    for (int64_t h = kTile; h < m && (sub <= 0 || h < sub); h *= 2) {
         int64_t q = 0;
         while ((2 * q + 1) * h < m) {
             GemmProb<T> pr[4], pq[4];
@@ -246,7 +250,7 @@ cudaError_t trtri_batched(const T* L, int64_t ldl, int64_t strideL, int64_t m, i
     template cudaError_t factor_column_block<T>(T*, int64_t, int64_t, RowSet<T>, RowSet<T>, T*,          \
                                                 int32_t*, int64_t, cudaStream_t, RowSet<T>);              \
     template cudaError_t trtri_batched<T>(const T*, int64_t, int64_t, int64_t, int64_t, T*, int64_t,     \
-                                          int64_t, T*, cudaStream_t, GemmFn<T>, void*);
+                                          int64_t, T*, cudaStream_t, GemmFn<T>, void*, int64_t);
 SGB_INST(double)
 SGB_INST(float)
 
