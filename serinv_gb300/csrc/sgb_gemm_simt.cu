@@ -8,6 +8,8 @@
 // and small tiles are what spreads the block-step GEMMs (512 x 512) over
 // all 152 SMs.  Operand tiles are staged through shared memory with
 // coalesced loads for either storage orientation.
+#include <string.h>
+
 #include "sgb_internal.cuh"
 
 namespace sgb {
@@ -379,6 +381,150 @@ __global__ void __launch_bounds__(NT) k_gemm_wide(const __grid_constant__ GemmLa
     }
 }
 
+// Launches with few output tiles.  An SM of this part issues one FP64 warp
+// instruction per 19 cycles, so a 32 x 32 tile of K = 64 runs for 20 us while
+// a block of b = 64 has only four of them for 152 SMs.  Tiles of 16 x 16 (or
+// 8 x 8 with k spread over four groups of threads) put the same product on 4
+// to 16 times as many SMs; 8 x 32 keeps a whole row of up to 32 columns in one
+// CTA for products in place.  128 threads, two outputs each; 64 k are staged
+// at a time, the next 64 on their way to registers meanwhile, so a product of
+// K <= 64 waits for memory once.
+constexpr int ST = 128, SKC = 64;
+
+template <typename T, int TM, int TN>
+__global__ void __launch_bounds__(ST) k_gemm_small(const __grid_constant__ GemmLaunch<T> L) {
+    constexpr int HN = TN / 2, G = ST / (TM * HN);  // thread columns; groups over k
+    constexpr int UA = TM * SKC / ST, UB = TN * SKC / ST;
+    __shared__ T As[SKC][TM + 1];
+    __shared__ T Bs[SKC][TN + 1];
+    const int tile = blockIdx.x;
+    int pi = 0;
+#pragma unroll 1
+    for (int q = 1; q < L.np; ++q)
+        if (tile >= L.p[q].tile_begin) pi = q;
+    const GemmProb<T>& P = L.p[pi];
+    int local = tile - P.tile_begin;
+    const int per_inst = P.tiles_m * P.tiles_n;
+    const int inst = local / per_inst;
+    local -= inst * per_inst;
+    const int tm = local / P.tiles_n, tn = local - tm * P.tiles_n;
+    const int m0 = tm * TM, n0 = tn * TN;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (P.lower_only && (n0 >> 5) > (m0 >> 5)) return;  // the 32 x 32 granularity of the other kernels
+
+    const int tid = threadIdx.x, g = tid / (TM * HN), o = tid % (TM * HN), r = o / HN, c = o % HN;
+    T acc0 = T(0), acc1 = T(0);
+#pragma unroll 1
+    for (int ti = 0; ti < P.nterms; ++ti) {
+        const GemmTerm<T>& t = P.term[ti];
+        const T* A = t.A + (int64_t)inst * t.strideA;
+        const T* B = t.B + (int64_t)inst * t.strideB;
+        int klo = 0, khi = t.K;
+        switch (t.kmode) {
+            case KM_GE_N0: klo = n0; break;
+            case KM_LT_N1: khi = min(t.K, n0 + TN); break;
+            case KM_GE_M0: klo = m0; break;
+            case KM_LT_M1: khi = min(t.K, m0 + TM); break;
+            default: break;
+        }
+        T ra[UA], rb[UB];
+        auto fetch = [&](int k0) {
+#pragma unroll
+            for (int u = 0; u < UA; ++u) {
+                const int e = tid + u * ST;
+                const int m = t.transA ? e % TM : e / SKC, k = t.transA ? e / TM : e % SKC;
+                const int gm = m0 + m, gk = k0 + k;
+                ra[u] = (gm < P.M && gk < khi) ? (t.transA ? A[(int64_t)gk * t.lda + gm] : A[(int64_t)gm * t.lda + gk])
+                                               : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < UB; ++u) {
+                const int e = tid + u * ST;
+                const int n = t.transB ? e / SKC : e % TN, k = t.transB ? e % SKC : e / TN;
+                const int gn = n0 + n, gk = k0 + k;
+                rb[u] = (gn < P.N && gk < khi) ? (t.transB ? B[(int64_t)gn * t.ldb + gk] : B[(int64_t)gk * t.ldb + gn])
+                                               : T(0);
+            }
+        };
+        if (klo < khi) fetch(klo);
+#pragma unroll 1
+        for (int k0 = klo; k0 < khi; k0 += SKC) {
+            __syncthreads();  // the previous slab's reads are done
+#pragma unroll
+            for (int u = 0; u < UA; ++u) {
+                const int e = tid + u * ST;
+                As[t.transA ? e / TM : e % SKC][t.transA ? e % TM : e / SKC] = ra[u];
+            }
+#pragma unroll
+            for (int u = 0; u < UB; ++u) {
+                const int e = tid + u * ST;
+                Bs[t.transB ? e % SKC : e / TN][t.transB ? e / SKC : e % TN] = rb[u];
+            }
+            __syncthreads();
+            if (k0 + SKC < khi) fetch(k0 + SKC);
+            const int kn = min(SKC, khi - k0);
+#pragma unroll 4
+            for (int k = g; k < kn; k += G) {
+                const T a = As[k][r];
+                acc0 = fma(a, Bs[k][c], acc0);
+                acc1 = fma(a, Bs[k][c + HN], acc1);
+            }
+        }
+    }
+    // the next launch may come in now (not earlier: its CTAs would settle beside
+    // this launch's and share the FP64 pipe of some SMs while others idle, which
+    // doubled a sweep's time at b = 256)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (G > 1) {  // the groups' sums, in the order of the groups
+        T* red = &As[0][0];
+        __syncthreads();
+        red[g * TM * TN + r * TN + c] = acc0;
+        red[g * TM * TN + r * TN + c + HN] = acc1;
+        __syncthreads();
+        if (g > 0) return;
+        for (int q = 1; q < G; ++q) {
+            acc0 += red[q * TM * TN + r * TN + c];
+            acc1 += red[q * TM * TN + r * TN + c + HN];
+        }
+    }
+    T* C = P.Cout + (int64_t)inst * P.strideC;
+    const T* Ci = P.Cin ? P.Cin + (int64_t)inst * P.strideCin : nullptr;
+    const int gm = m0 + r;
+    if (gm >= P.M) return;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int gn = n0 + c + j * HN;
+        if (gn >= P.N) continue;
+        T v = P.alpha * (j ? acc1 : acc0);
+        if (Ci != nullptr && P.beta != T(0)) {
+            const T x = P.transCin ? Ci[(int64_t)gn * P.ldcin + gm] : Ci[(int64_t)gm * P.ldcin + gn];
+            v = fma(P.beta, x, v);
+        }
+        C[(int64_t)gm * P.ldc + gn] = v;
+    }
+}
+
+template <typename T, int TM, int TN>
+cudaError_t launch_small(const GemmLaunch<T>& L, unsigned grid, cudaStream_t s) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(ST);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    memset(&at, 0, sizeof(at));
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    // Brought in while its predecessor leaves, unless the FP64 pipe would feel
+    // where its CTAs settle: they then share some SMs while others idle.  FP64
+    // selected inverse at b = 256 (288 CTAs a launch) 29.2 ms so against 16.0
+    // in stream order, at b = 180 (156 CTAs) 1.68 against 1.55, at b = 64 (80
+    // CTAs) 1.55 against 2.09; FP32 at b = 130 (99 CTAs) 1.01 against 1.47.
+    cfg.numAttrs = (sizeof(T) == 4 || grid <= 80) ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_gemm_small<T, TM, TN>, L);
+}
+
 inline void launch_wide(const GemmLaunch<float>& L, unsigned grid, cudaStream_t s) {
     k_gemm_wide<<<grid, NT, 0, s>>>(L);
 }
@@ -431,6 +577,92 @@ bool skinny_ok(const GemmProb<T>* probs, int np) {
     return any;
 }
 
+// Which kernel's tiles a launch gets.
+enum Shape { SH_SIMT, SH_WIDE, SH_SKINNY, SH_16, SH_8, SH_ROWS };
+struct Tile {
+    int m, n;
+};
+constexpr Tile kTiles[] = {{BM, BN}, {WB, WB}, {SK_ROWS, 1 << 30}, {16, 16}, {8, 8}, {8, 32}};
+constexpr int64_t kSms = 152;
+
+template <typename T>
+int64_t count_tiles(const GemmProb<T>* probs, int np, Tile t) {
+    int64_t n = 0;
+    for (int i = 0; i < np; ++i)
+        if (probs[i].M > 0 && probs[i].N > 0 && probs[i].batch > 0)
+            n += ceil_div(probs[i].M, t.m) * ceil_div(probs[i].N, t.n) * probs[i].batch;
+    return n;
+}
+
+// Whether operand X (rows x cols, leading dimension ld) may share elements
+// with the M x N output of p.  Two sets of columns of one row-major array are
+// apart although their byte ranges interleave.
+template <typename T>
+bool overlaps(const GemmProb<T>& p, const T* X, int64_t rows, int64_t cols, int64_t ld, int64_t stride) {
+    if (rows <= 0 || cols <= 0) return false;
+    uintptr_t clo, chi, lo, hi;
+    span(p.Cout, p.M, p.N, p.ldc, p.strideC, p.batch, clo, chi);
+    span(X, rows, cols, ld, stride, p.batch, lo, hi);
+    if (hi <= clo || chi <= lo) return false;
+    const int64_t bytes = (int64_t)((uintptr_t)X - (uintptr_t)p.Cout);
+    if (ld != p.ldc || bytes % (int64_t)sizeof(T) != 0) return true;
+    if (p.batch > 1 && (stride % ld != 0 || p.strideC % ld != 0)) return true;
+    int64_t off = bytes / (int64_t)sizeof(T) % ld;
+    if (off < 0) off += ld;
+    return off < p.N || off + cols > ld;
+}
+
+// 0: no operand overlaps its problem's output; 1: some do, and a tile of 32
+// columns holds their whole rows; 2: otherwise.
+template <typename T>
+int in_place(const GemmProb<T>* probs, int np) {
+    int worst = 0;
+    for (int i = 0; i < np; ++i) {
+        const GemmProb<T>& p = probs[i];
+        if (p.M <= 0 || p.N <= 0 || p.batch <= 0) continue;
+        bool over = p.Cin != nullptr && p.transCin;
+        for (int t = 0; t < p.nterms; ++t) {
+            const GemmTerm<T>& g = p.term[t];
+            over = over || overlaps<T>(p, g.A, g.transA ? g.K : p.M, g.transA ? p.M : g.K, g.lda, g.strideA) ||
+                   overlaps<T>(p, g.B, g.transB ? p.N : g.K, g.transB ? g.K : p.N, g.ldb, g.strideB);
+        }
+        if (over) worst = p.N <= 32 && worst < 2 ? 1 : 2;
+    }
+    return worst;
+}
+
+// Time of a launch on FP64: the tiles an SM gets, times a tile's outputs (each
+// k of an output is an FMA on its pipe).  b = 64 with a = 16: 80 tiles of 8 x 8
+// count 64, 20 of 16 x 16 count 256, 6 of 32 x 32 count 1024, and the back-sweep's
+// launch takes 10 us with the first against 31 us with the last; b = 256 with
+// a = 32: 288 tiles of 16 x 16 count 512 against 1024, 62 against 114 us.  From
+// b = 512 on the three agree and the larger tile reads less.
+// FP32 has the arithmetic for any tile; the smaller one is taken while the
+// larger leaves a third of the SMs without work (b = 130: 10 against 18 us).
+template <typename T>
+Shape pick(const GemmProb<T>* probs, int np) {
+    if (skinny_ok<T>(probs, np)) return SH_SKINNY;
+    const Shape big = wide_ok<T>(probs, np) ? SH_WIDE : SH_SIMT;
+    const int ip = in_place<T>(probs, np);
+    if (ip == 2) return big;
+    auto waves = [&](Shape h) { return ceil_div(count_tiles<T>(probs, np, kTiles[h]), kSms); };
+    if (ip == 1) return count_tiles<T>(probs, np, kTiles[SH_ROWS]) <= 4 * kSms ? SH_ROWS : SH_SIMT;
+    if (sizeof(T) == 4) {
+        if (count_tiles<T>(probs, np, kTiles[big]) * 3 >= kSms * 2) return big;
+        return count_tiles<T>(probs, np, kTiles[SH_16]) * 3 >= kSms * 2 ? SH_16 : SH_8;
+    }
+    Shape best = big;
+    int64_t cost = waves(big) * BM * BN;
+    for (Shape h : {SH_16, SH_8}) {
+        const int64_t c = waves(h) * kTiles[h].m * kTiles[h].n;
+        if (c < cost) {
+            best = h;
+            cost = c;
+        }
+    }
+    return best;
+}
+
 }  // namespace
 
 template <typename T>
@@ -469,14 +701,13 @@ cudaError_t gemm_simt(GemmProb<T>* probs, int np, cudaStream_t s) {
     GemmLaunch<T> L;
     L.np = 0;
     int64_t total = 0;
-    const bool skinny = skinny_ok<T>(probs, np);
-    const bool wide = !skinny && wide_ok<T>(probs, np);
-    const int tile_m = skinny ? SK_ROWS : (wide ? WB : BM);
+    const Shape shape = pick<T>(probs, np);
+    const Tile tile = kTiles[shape];
     for (int i = 0; i < np; ++i) {
         GemmProb<T> p = probs[i];
         if (p.M <= 0 || p.N <= 0 || p.batch <= 0) continue;
-        p.tiles_m = (int32_t)ceil_div(p.M, tile_m);
-        p.tiles_n = skinny ? 1 : (int32_t)ceil_div(p.N, wide ? WB : BN);
+        p.tiles_m = (int32_t)ceil_div(p.M, tile.m);
+        p.tiles_n = (int32_t)ceil_div(p.N, tile.n);
         p.tile_begin = (int32_t)total;
         total += (int64_t)p.tiles_m * p.tiles_n * p.batch;
         L.p[L.np++] = p;
@@ -488,11 +719,17 @@ cudaError_t gemm_simt(GemmProb<T>* probs, int np, cudaStream_t s) {
     double fl = 0.0;
     for (int i = 0; i < L.np; ++i) fl += useful_flops<T>(L.p[i]);
     prof_before(s, SGB_KCLASS_GEMM);
-    if (skinny) k_gemm_skinny<T><<<(unsigned)total, NT, 0, s>>>(L);
-    else if (wide) launch_wide(L, (unsigned)total, s);
-    else k_gemm_simt<T><<<(unsigned)total, NT, 0, s>>>(L);
+    cudaError_t e = cudaSuccess;
+    switch (shape) {
+        case SH_SKINNY: k_gemm_skinny<T><<<(unsigned)total, NT, 0, s>>>(L); break;
+        case SH_WIDE: launch_wide(L, (unsigned)total, s); break;
+        case SH_16: e = launch_small<T, 16, 16>(L, (unsigned)total, s); break;
+        case SH_8: e = launch_small<T, 8, 8>(L, (unsigned)total, s); break;
+        case SH_ROWS: e = launch_small<T, 8, 32>(L, (unsigned)total, s); break;
+        default: k_gemm_simt<T><<<(unsigned)total, NT, 0, s>>>(L); break;
+    }
     prof_after(SGB_KCLASS_GEMM, s, fl);
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 template cudaError_t gemm_simt<double>(GemmProb<double>*, int, cudaStream_t);

@@ -349,10 +349,9 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
     const int64_t m = a.m;
     const int64_t nt = (m + kTile - 1) / kTile;
     const int tx = tid & 31, ty = tid >> 5;
-    // the next kernel in the stream (a programmatic dependent launch) may
-    // start launching now; it waits for this grid's completion before it
-    // touches memory
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // A dependent launch comes in as this grid's CTAs leave: let in at the
+    // start, its CTAs settled on a few SMs while this grid held one CTA of every
+    // SM, and the product after an FP32 panel at b = 130 took 8 us longer.
     unsigned* F = a.bar + 0;
     unsigned* I = a.bar + 1;
     unsigned* barB = a.bar + 4;
@@ -376,7 +375,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
             const int64_t c0 = p * kTile;
             const int w = tile_w(p);
             if (p >= 3 && !wait_count(I, (unsigned)(p - 2), a.status, &S.flag, a.spin)) return;  // buffer p % 3 free
-            const int buf = (int)(p % 3);
+                const int buf = (int)(p % 3);
             // tile p >= 1 arrives by value from the helpers (their update
             // with column block p-1); tile-row staging p-1 is then free
             factor_tile_m<T>(S, a.diag + c0 * a.ldd + c0, a.ldd, w, a.info, a.row0 + c0, Mg + buf * kTile * kTile,
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
         for (int64_t p = 0; p < nt; ++p) {
             const int64_t c0 = p * kTile;
             const int w = tile_w(p);
-            if (!wait_count(F, (unsigned)(p + 1), a.status, &S.flag, a.spin)) return;
+                if (!wait_count(F, (unsigned)(p + 1), a.status, &S.flag, a.spin)) return;
             const int buf = (int)(p % 3);
             {
                 const T* mt = Mg + buf * kTile * kTile;
