@@ -75,6 +75,28 @@ int parse_inv_slices(int precision, int S) {
     return (precision >> 16) & 0xff;
 }
 
+// FP64 arithmetic of pobtaf's Schur products and of pobtasi on the tensor
+// cores: kExactSlices slices (63 bits below each row's largest entry, level
+// sums added as integers, one rounding to FP64 per element).  Against 64 bits
+// the selected inverse is 8.2e-16 .. 1.4e-15 off at n=32 b=512 a=64 where the
+// FP64 pipe's sums are 9.0e-16 .. 1.5e-15 off, the factor is the same, and with
+// rows and columns scaled by up to 10^+-6 neither changes (the products over
+// rows of an inverse are balanced by its diagonal).  The factorization of the
+// column blocks stays on the FP64 pipe.
+// Below the lines the slicing and the longer epilogue cost more than the FP64
+// pipe's 16 x 16 tiles: selected inverse n=64 (us) b=208 4961 against 4617, b=224
+// 4574 / 5458, b=256 a=32 5561 / 8055, b=512 (n=32) 5618 / 26456; factorization
+// b=224 8787 / 8552, b=240 9441 / 10090, b=512 (n=32) 13522 / 16960.
+constexpr int64_t kExactMinFactor = 240, kExactMinInverse = 224;
+
+// The slice count of a native FP64 sweep, or 0: the FP64 pipe.
+int exact_slices(const sgb_bta* m, bool inverse) {
+    return m->dtype == SGB_F64 && m->b >= (inverse ? kExactMinInverse : kExactMinFactor) &&
+                   ceil_div(m->b, 32) * 32 <= kTcMaxK
+               ? kExactSlices
+               : 0;
+}
+
 // Everything a block sweep needs besides the matrix: precision and the
 // tensor-core scratch carved from the caller's workspace.
 struct Ctx {
@@ -240,7 +262,7 @@ struct PobtafWs {
         tc_bytes = S ? tc_bound(Sm, mx, m->b, 4) : 0;  // up to four problems per product launch
         tc = c.take(tc_bytes);
         // mixed precision only: L_ii^{-T} of the current diagonal block
-        xinv = c.take(S ? sizeof(T) * m->b * m->b : 0);
+        xinv = c.take(S && S <= 7 ? sizeof(T) * m->b * m->b : 0);
         total = c.off;
     }
 };
@@ -310,6 +332,24 @@ struct PobtasWs {
     }
 };
 
+// Workspace of a sweep, and the slices it runs with: a native FP64 call takes
+// the exact slice products when the workspace it was given has room for them
+// (the size queries ask for it) and the FP64 pipe otherwise.
+size_t taf_bytes(const sgb_bta* m, int S, int Si) {
+    return m->dtype == SGB_F64 ? PobtafWs<double>(m, S, Si).total : PobtafWs<float>(m, S, Si).total;
+}
+size_t tasi_bytes(const sgb_bta* m, int S, int Si, int64_t cap = kSiChunk) {
+    return m->dtype == SGB_F64 ? PobtasiWs<double>(m, S, Si, cap).total : PobtasiWs<float>(m, S, Si, cap).total;
+}
+int taf_slices(const sgb_bta* m, int S, size_t have) {
+    const int X = S ? 0 : exact_slices(m, false);
+    return X && have >= taf_bytes(m, X, 0) ? X : S;
+}
+int tasi_slices(const sgb_bta* m, int S, size_t have) {
+    const int X = S ? 0 : exact_slices(m, true);
+    return X && have >= tasi_bytes(m, X, 0) ? X : S;
+}
+
 int check_ws(void* ws, size_t have, size_t need) {
     if (need == 0) return SGB_OK;
     if (ws == nullptr || have < need) return SGB_ERR_WORKSPACE;
@@ -338,6 +378,14 @@ void set_term(GemmProb<T>& p, int t, const T* A, int64_t lda, int transA, const 
     p.term[t].K = (int32_t)K;
     p.term[t].kmode = (int8_t)kmode;
     if (t + 1 > p.nterms) p.nterms = t + 1;
+}
+
+// Contraction over the rows of an SPD inverse X: balanced by its diagonal.
+template <typename T>
+void balance(GemmProb<T>& p, int t, const T* X, int64_t ld) {
+    p.term[t].ks = X;
+    p.term[t].ldks = ld + 1;
+    p.term[t].ksmode = KS_SPD_DIAG;
 }
 
 // Copy problem: Cout = Cin (M x N).
@@ -852,6 +900,8 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
     cx.status = (int32_t*)(base + W.status);
     Ctx cxi = cx;  // the inversions and the products with L_ii^{-1}
     cxi.slices = Si ? Si : S;
+    Ctx cxt = cxi;  // the tip: too small for the exact slices to pay
+    if (S > 7) cxt.slices = 0;
     T* Linv = (T*)(base + W.linv);
     T* Ltinv = (T*)(base + W.linv_tip);
     T* trs = (T*)(base + W.trtri);
@@ -864,13 +914,13 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
     }
     if (invert_last_block && a) {
         // X_T = L_T^{-T} L_T^{-1}  (:115-119)
-        SGB_TRY(trtri_run<T>(cxi, Tp, a, 1, Ltinv, trs, s));
+        SGB_TRY(trtri_run<T>(cxt, Tp, a, 1, Ltinv, trs, s));
         GemmProb<T> p = prob<T>();
         p.M = p.N = (int32_t)a;
         set_term<T>(p, 0, Ltinv, a, 1, Ltinv, a, 0, a, KM_GE_M0);
         p.Cout = Tp;
         p.ldc = a;
-        SGB_TRY(run_gemm<T>(cxi, &p, 1, s));
+        SGB_TRY(run_gemm<T>(cxt, &p, 1, s));
     }
     if (hl) SGB_TRY(hl->give_tip());
 
@@ -940,7 +990,11 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 GemmProb<T> p = prob<T>();
                 p.M = p.N = (int32_t)b;
                 set_term<T>(p, 0, B.d(i + 1), b, 0, G, b, 0, b);
-                if (a) set_term<T>(p, 1, B.ar(i + 1), b, 1, H, b, 0, a);
+                balance<T>(p, 0, B.d(i + 1), b);
+                if (a) {
+                    set_term<T>(p, 1, B.ar(i + 1), b, 1, H, b, 0, a);
+                    balance<T>(p, 1, Tp, a);
+                }
                 p.alpha = T(-1);
                 p.Cout = B.lo(i);
                 p.ldc = b;
@@ -951,8 +1005,12 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 p.M = (int32_t)a;
                 p.N = (int32_t)b;
                 int t = 0;
-                if (has_next) set_term<T>(p, t++, B.ar(i + 1), b, 0, G, b, 0, b);
+                if (has_next) {
+                    set_term<T>(p, t, B.ar(i + 1), b, 0, G, b, 0, b);
+                    balance<T>(p, t++, B.d(i + 1), b);
+                }
                 set_term<T>(p, t, Tp, a, 0, H, b, 0, a);
+                balance<T>(p, t, Tp, a);
                 p.alpha = T(-1);
                 p.Cout = B.ar(i);
                 p.ldc = b;
@@ -964,8 +1022,14 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 GemmProb<T> p = prob<T>();
                 p.M = p.N = (int32_t)b;
                 int t = 0;
-                if (has_next) set_term<T>(p, t++, B.lo(i), b, 1, G, b, 0, b);
-                if (a) set_term<T>(p, t++, B.ar(i), b, 1, H, b, 0, a);
+                if (has_next) {
+                    set_term<T>(p, t, B.lo(i), b, 1, G, b, 0, b);
+                    balance<T>(p, t++, B.d(i + 1), b);
+                }
+                if (a) {
+                    set_term<T>(p, t, B.ar(i), b, 1, H, b, 0, a);
+                    balance<T>(p, t++, Tp, a);
+                }
                 p.alpha = T(-1);
                 p.beta = T(1);
                 p.Cin = B.d(i);
@@ -1511,6 +1575,13 @@ bool item_keeps_inverses(const sgb_bta* m, int precision, int ops) {
 
 }  // namespace
 
+int pobtaf_least_workspace(const sgb_bta* m, size_t* bytes) {
+    if (cx_dtype(m)) return sgb_pobtaf_workspace_size(m, SGB_PREC_NATIVE, bytes);
+    const int rc = check_bta(m);
+    if (rc == SGB_OK) *bytes = taf_bytes(m, 0, 0);
+    return rc;
+}
+
 size_t plan_item_ws(const sgb_bta* m, int ops, int precision, int64_t nrhs) {
     size_t need = 0, x = 0;
     if (ops & SGB_OP_POBTAF) {
@@ -1615,8 +1686,10 @@ sgb_bta ring_desc(const sgb_bta* host, char* ws, const StreamWs& L) {
     return d;
 }
 
-int stream_sizes(const sgb_bta* host, int precision, int64_t ring, bool inverse, int64_t* R, size_t* sweep,
-                 size_t* total) {
+// *S receives the slices the sweep runs with: the exact products of a native
+// FP64 call if `have` bytes hold them (SIZE_MAX: the query).
+int stream_sizes(const sgb_bta* host, int precision, int64_t ring, bool inverse, size_t have, int* slices, int64_t* R,
+                 size_t* sweep, size_t* total) {
     int rc = check_bta(host);
     if (rc) return rc;
     const int S = parse_precision(precision, host->dtype);
@@ -1624,12 +1697,12 @@ int stream_sizes(const sgb_bta* host, int precision, int64_t ring, bool inverse,
     const int Si = parse_inv_slices(precision, S);
     *R = inverse ? ring_slots(ring, kRingPobtasi, true) : ring_slots(ring, kRingPobtaf, false);
     if (*R < 2 || *R > ((int64_t)1 << 20)) return SGB_ERR_SHAPE;
-    if (inverse)
-        *sweep = host->dtype == SGB_F64 ? PobtasiWs<double>(host, S, Si, *R / 2).total
-                                        : PobtasiWs<float>(host, S, Si, *R / 2).total;
-    else
-        *sweep = host->dtype == SGB_F64 ? PobtafWs<double>(host, S, Si).total : PobtafWs<float>(host, S, Si).total;
-    *total = StreamWs(host, *sweep, *R).total;
+    for (int X : {S ? S : exact_slices(host, inverse), S}) {
+        *slices = X;
+        *sweep = inverse ? tasi_bytes(host, X, Si, *R / 2) : taf_bytes(host, X, Si);
+        *total = StreamWs(host, *sweep, *R).total;
+        if (have >= *total) break;
+    }
     return SGB_OK;
 }
 
@@ -1667,7 +1740,8 @@ int sgb_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes) {
     if (S < 0) return -S;
     if (!bytes) return SGB_ERR_ARG;
     const int Si = parse_inv_slices(precision, S);
-    *bytes = m->dtype == SGB_F64 ? PobtafWs<double>(m, S, Si).total : PobtafWs<float>(m, S, Si).total;
+    *bytes = m->dtype == SGB_F64 ? PobtafWs<double>(m, S ? S : exact_slices(m, false), Si).total
+                                 : PobtafWs<float>(m, S, Si).total;
     return SGB_OK;
 }
 
@@ -1679,7 +1753,8 @@ int sgb_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes) {
     if (S < 0) return -S;
     if (!bytes) return SGB_ERR_ARG;
     const int Si = parse_inv_slices(precision, S);
-    *bytes = m->dtype == SGB_F64 ? PobtasiWs<double>(m, S, Si).total : PobtasiWs<float>(m, S, Si).total;
+    *bytes = m->dtype == SGB_F64 ? PobtasiWs<double>(m, S ? S : exact_slices(m, true), Si).total
+                                 : PobtasiWs<float>(m, S, Si).total;
     return SGB_OK;
 }
 
@@ -1765,14 +1840,13 @@ int sgb_pobtaf(const sgb_bta* m, int factorize_last_block, int precision, void* 
     if (rc) return rc;
     const int S = parse_precision(precision, m->dtype);
     if (S < 0) return -S;
-    size_t need = 0;
-    sgb_pobtaf_workspace_size(m, precision, &need);
-    if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
+    const int Si = parse_inv_slices(precision, S);
+    if ((rc = check_ws(workspace, workspace_bytes, taf_bytes(m, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
     SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
-    const int Si = parse_inv_slices(precision, S);
-    if (m->dtype == SGB_F64) return pobtaf_run<double>(m, factorize_last_block, S, Si, workspace, info, s);
+    if (m->dtype == SGB_F64)
+        return pobtaf_run<double>(m, factorize_last_block, taf_slices(m, S, workspace_bytes), Si, workspace, info, s);
     return pobtaf_run<float>(m, factorize_last_block, S, Si, workspace, info, s);
 }
 
@@ -1785,13 +1859,12 @@ int sgb_pobtasi(const sgb_bta* m, int invert_last_block, int precision, void* wo
     if (rc) return rc;
     const int S = parse_precision(precision, m->dtype);
     if (S < 0) return -S;
-    size_t need = 0;
-    sgb_pobtasi_workspace_size(m, precision, &need);
-    if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
+    const int Si = parse_inv_slices(precision, S);
+    if ((rc = check_ws(workspace, workspace_bytes, tasi_bytes(m, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
-    const int Si = parse_inv_slices(precision, S);
-    if (m->dtype == SGB_F64) return pobtasi_run<double>(m, invert_last_block, S, Si, workspace, s);
+    if (m->dtype == SGB_F64)
+        return pobtasi_run<double>(m, invert_last_block, tasi_slices(m, S, workspace_bytes), Si, workspace, s);
     return pobtasi_run<float>(m, invert_last_block, S, Si, workspace, s);
 }
 
@@ -1971,9 +2044,8 @@ int sgb_pobtaf_host(const sgb_bta* host, const sgb_bta* dev, int factorize_last_
     if (rc) return rc;
     const int S = parse_precision(precision, dev->dtype);
     if (S < 0) return -S;
-    size_t need = 0;
-    sgb_pobtaf_workspace_size(dev, precision, &need);
-    if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
+    const int Si = parse_inv_slices(precision, S);
+    if ((rc = check_ws(workspace, workspace_bytes, taf_bytes(dev, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
     SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
@@ -1982,37 +2054,39 @@ int sgb_pobtaf_host(const sgb_bta* host, const sgb_bta* dev, int factorize_last_
     hl.d = dev;
     hl.ascending = true;
     hl.es = dev->dtype == SGB_F64 ? 8 : 4;
-    const int Si = parse_inv_slices(precision, S);
     if (dev->dtype == SGB_F64)
-        return pobtaf_run<double>(dev, factorize_last_block, S, Si, workspace, info, s, &hl);
+        return pobtaf_run<double>(dev, factorize_last_block, taf_slices(dev, S, workspace_bytes), Si, workspace, info, s,
+                                  &hl);
     return pobtaf_run<float>(dev, factorize_last_block, S, Si, workspace, info, s, &hl);
 }
 
 int sgb_pobtaf_stream_workspace_size(const sgb_bta* host, int precision, int64_t ring, size_t* bytes) {
     if (cx_dtype(host)) return SGB_ERR_UNSUPPORTED;
     if (!bytes) return SGB_ERR_ARG;
+    int S = 0;
     int64_t R = 0;
     size_t sweep = 0;
-    return stream_sizes(host, precision, ring, false, &R, &sweep, bytes);
+    return stream_sizes(host, precision, ring, false, SIZE_MAX, &S, &R, &sweep, bytes);
 }
 
 int sgb_pobtasi_stream_workspace_size(const sgb_bta* host, int precision, int64_t ring, size_t* bytes) {
     if (cx_dtype(host)) return SGB_ERR_UNSUPPORTED;
     if (!bytes) return SGB_ERR_ARG;
+    int S = 0;
     int64_t R = 0;
     size_t sweep = 0;
-    return stream_sizes(host, precision, ring, true, &R, &sweep, bytes);
+    return stream_sizes(host, precision, ring, true, SIZE_MAX, &S, &R, &sweep, bytes);
 }
 
 int sgb_pobtaf_stream(const sgb_bta* host, int factorize_last_block, int precision, int64_t ring, void* workspace,
                       size_t workspace_bytes, int32_t* info, void* stream) {
     if (cx_dtype(host)) return SGB_ERR_UNSUPPORTED;
+    int S = 0;
     int64_t R = 0;
     size_t sweep = 0, total = 0;
-    int rc = stream_sizes(host, precision, ring, false, &R, &sweep, &total);
+    int rc = stream_sizes(host, precision, ring, false, workspace_bytes, &S, &R, &sweep, &total);
     if (rc) return rc;
     if ((rc = check_ws(workspace, workspace_bytes, total))) return rc;
-    const int S = parse_precision(precision, host->dtype);
     const int Si = parse_inv_slices(precision, S);
     const StreamWs L(host, sweep, R);
     const sgb_bta dm = ring_desc(host, (char*)workspace, L);
@@ -2037,12 +2111,12 @@ int sgb_pobtaf_stream(const sgb_bta* host, int factorize_last_block, int precisi
 int sgb_pobtasi_stream(const sgb_bta* host, int invert_last_block, int precision, int64_t ring, void* workspace,
                        size_t workspace_bytes, void* stream) {
     if (cx_dtype(host)) return SGB_ERR_UNSUPPORTED;
+    int S = 0;
     int64_t R = 0;
     size_t sweep = 0, total = 0;
-    int rc = stream_sizes(host, precision, ring, true, &R, &sweep, &total);
+    int rc = stream_sizes(host, precision, ring, true, workspace_bytes, &S, &R, &sweep, &total);
     if (rc) return rc;
     if ((rc = check_ws(workspace, workspace_bytes, total))) return rc;
-    const int S = parse_precision(precision, host->dtype);
     const int Si = parse_inv_slices(precision, S);
     const StreamWs L(host, sweep, R);
     const sgb_bta dm = ring_desc(host, (char*)workspace, L);
@@ -2069,9 +2143,8 @@ int sgb_pobtasi_host(const sgb_bta* host, const sgb_bta* dev, int invert_last_bl
     if (rc) return rc;
     const int S = parse_precision(precision, dev->dtype);
     if (S < 0) return -S;
-    size_t need = 0;
-    sgb_pobtasi_workspace_size(dev, precision, &need);
-    if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
+    const int Si = parse_inv_slices(precision, S);
+    if ((rc = check_ws(workspace, workspace_bytes, tasi_bytes(dev, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
     HostLink hl;
@@ -2079,8 +2152,8 @@ int sgb_pobtasi_host(const sgb_bta* host, const sgb_bta* dev, int invert_last_bl
     hl.d = dev;
     hl.ascending = false;
     hl.es = dev->dtype == SGB_F64 ? 8 : 4;
-    const int Si = parse_inv_slices(precision, S);
-    if (dev->dtype == SGB_F64) return pobtasi_run<double>(dev, invert_last_block, S, Si, workspace, s, &hl);
+    if (dev->dtype == SGB_F64)
+        return pobtasi_run<double>(dev, invert_last_block, tasi_slices(dev, S, workspace_bytes), Si, workspace, s, &hl);
     return pobtasi_run<float>(dev, invert_last_block, S, Si, workspace, s, &hl);
 }
 

@@ -21,6 +21,15 @@
 // stores FP64: two FP64 instructions per element, because every FP64 warp
 // instruction occupies its SM quarter for ~64 cycles on this part.
 //
+// S = 9 (kExactSlices) stands in for FP64 arithmetic: 63 bits below the row
+// maximum, seven accumulators (levels 0..5 and the rest), the level sums added
+// as integers and rounded once to FP64, and the contraction index balanced by a
+// power of two per k where the caller names a diagonal (GemmTerm::ks): an
+// inverse's columns and the rows they meet may differ by any factor, and a
+// fixed-point row keeps only what lies 63 bits below its largest entry.  One
+// 576 x 512 x 512 launch with 45 slice pairs against 21 at S = 6: 42 us
+// against 31, and its operands' slicing 22 against 16 us.
+//
 // This is the published Ozaki error-free splitting idea (Ozaki, Ogita,
 // Oishi, Rump) specialised to fixed-point digits and level-grouped exact
 // tensor-core accumulation.
@@ -71,6 +80,9 @@ struct SplitSrc {
     int64_t ld_r, ld_k;   // element (r, k) at X[r*ld_r + k*ld_k]
     int64_t stride;       // batch stride (elements)
     int32_t K, koff;      // source K extent; destination K offset (multiple of TC_BK)
+    const double* ks;     // balance of k (GemmTerm::ks), or null
+    int64_t ldks, ks_stride;
+    int32_t ksign, kshift;  // k's elements are scaled by 2^(ksign * (exponent of ks >> kshift))
 };
 
 // One operand of one problem: the rows of op(A) (or the columns of op(B))
@@ -79,7 +91,8 @@ struct SplitJob {
     SplitSrc src[2];
     int32_t nsrc;
     __nv_bfloat16* out;   // per instance: [S][Rpad/RT][Kpad/32] chunks of RT x 32 (core-matrix order)
-    int32_t* exps;        // [Rpad] per instance (biased FP64 exponent of the row max, 0 for a zero row)
+    int32_t* exps;        // [Rpad] per instance: kExpBias + biased FP64 exponent of the row max, 0 for a zero
+                          // row, kExpNan for a row that holds an Inf or NaN
     int64_t out_stride, exp_stride;
     int32_t R, Rpad, Kpad;
     int32_t RT;           // rows per chunk: 128 for A, the tile width for B
@@ -87,6 +100,8 @@ struct SplitJob {
     int32_t strips, strip_begin;  // kSplitRows-row strips per instance; first CTA of the job
 };
 
+constexpr int kExpBias = 8192;  // keeps a scaled exponent positive
+constexpr int kExpNan = -1;
 constexpr int kSplitRows = 8;
 constexpr int kSplitThreads = 512;  // two CTAs per SM, eight warps per scheduler: latency bound
 constexpr int kSplitLd = kTcMaxK + 1;  // odd stride: conflict-free row and column access
@@ -105,37 +120,50 @@ __device__ __forceinline__ int find_job(const SplitLaunch& L, int cta) {
     return ji;
 }
 
-// Balanced base-128 digits of x scaled by the row exponent Erow (biased).
+// Balanced base-128 digits of x 2^sk scaled by the row exponent Erow (biased).
 template <int S>
-__device__ __forceinline__ void digits(double x, int Erow, int (&d)[S]) {
+__device__ __forceinline__ void digits(double x, int sk, int Erow, int (&d)[S]) {
     const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
     const int Ex = (int)((bits >> 52) & 0x7ff);
 #pragma unroll
     for (int p = 0; p < S; ++p) d[p] = 0;
-    if (Ex == 0 || Erow == 0) return;  // zero, subnormal (flushed) or zero row
+    if (Ex == 0) return;  // zero or subnormal (flushed)
     const long long m = (long long)((bits & ((1ull << 52) - 1)) | (1ull << 52));
-    const int rs = Erow - Ex + 53 - 7 * S;  // right shift; >= 53 - 7S > 0 for S <= 7
+    const int rs = Erow - (Ex + sk) + 53 - 7 * S;  // right shift (for S > 7 also a left shift)
     long long X;
     if (rs >= 62) X = 0;
     else if (rs <= 0) X = m << (-rs);
     else X = (m + (1ll << (rs - 1))) >> rs;
     if (bits >> 63) X = -X;
-    // |X| < 2^(7S+1) <= 2^50: the low L digits come out of the low 7L bits
-    // and the rest out of the high part, all in 32-bit arithmetic (the
-    // balanced digit v = ((x mod 128) ^ 64) - 64 lies in [-64, 63]; removing
-    // the low digits leaves a carry of 0 or 1 for the high part).
+    // |X| < 2^(7S+1) (2^63 for S = 9: a 53-bit integer shifted left): the low
+    // digits come out of limbs of up to three digits in 32-bit arithmetic (the
+    // balanced digit v = ((x mod 128) ^ 64) - 64 lies in [-64, 63]; removing the
+    // digits of a limb leaves a carry of 0 or 1 for the next).
     constexpr int L = (S - 1) < 3 ? (S - 1) : 3;
     int lo = (int)(X & ((1ll << (7 * L)) - 1));
-    int hi = (int)(X >> (7 * L));
+    X >>= 7 * L;
 #pragma unroll
     for (int p = S - 1; p >= S - L; --p) {
         const int v = ((lo & 127) ^ 64) - 64;
         d[p] = v;
         lo = (lo - v) >> 7;
     }
-    hi += lo;
+    X += lo;
+    if constexpr (S > 7) {
+        int mid = (int)(X & ((1ll << 21) - 1));
+        X >>= 21;
 #pragma unroll
-    for (int p = S - L - 1; p >= 1; --p) {
+        for (int p = S - L - 1; p >= S - L - 3; --p) {
+            const int v = ((mid & 127) ^ 64) - 64;
+            d[p] = v;
+            mid = (mid - v) >> 7;
+        }
+        X += mid;
+    }
+    constexpr int P0 = S > 7 ? S - L - 3 : S - L;  // digits left
+    int hi = (int)X;
+#pragma unroll
+    for (int p = P0 - 1; p >= 1; --p) {
         const int v = ((hi & 127) ^ 64) - 64;
         d[p] = v;
         hi = (hi - v) >> 7;
@@ -163,6 +191,8 @@ template <int S>
 __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__ SplitLaunch L) {
     __shared__ double t[kSplitRows][kSplitLd];
     __shared__ int ex[kSplitRows];
+    constexpr bool kScaled = S > 7;
+    __shared__ short sk[kScaled ? kTcMaxK : 1];  // power of two of each k
     pdl_enter();
     const SplitJob& J = L.j[find_job(L, blockIdx.x)];
     const int local = blockIdx.x - J.strip_begin;
@@ -179,6 +209,17 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
         const SplitSrc& src = J.src[q];
         const double* X = src.X + (int64_t)inst * src.stride;
         const int Kp = (src.K + TC_BK - 1) / TC_BK * TC_BK;
+        if constexpr (kScaled) {
+            const double* ks = src.ks ? src.ks + (int64_t)inst * src.ks_stride : nullptr;
+            for (int k = tid; k < Kp; k += kSplitThreads) {
+                int e = 0;
+                if (ks != nullptr && k < src.K) {
+                    const int eb = (int)(((unsigned long long)__double_as_longlong(ks[(int64_t)k * src.ldks]) >> 52) & 0x7ff);
+                    if (eb != 0 && eb != 0x7ff) e = src.ksign * ((eb - 1023) >> src.kshift);
+                }
+                sk[src.koff + k] = (short)e;
+            }
+        }
         if (src.ld_k == 1) {
             constexpr int KU = (kTcMaxK + kSplitThreads - 1) / kSplitThreads;  // 2
             double v[kSplitRows][KU];
@@ -213,20 +254,33 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
             }
         }
     }
-    if (J.nsrc == 0)
+    if (J.nsrc == 0) {
         for (int e = tid; e < kSplitRows * J.Kpad; e += kSplitThreads) t[e / J.Kpad][e % J.Kpad] = 0.0;
+        if (kScaled)
+            for (int e = tid; e < J.Kpad; e += kSplitThreads) sk[e] = 0;
+    }
     __syncthreads();
     const int warp = tid >> 5, lane = tid & 31;
     if (warp < kSplitRows) {
-        int emax = 0;
+        int emax = 0, bad = 0;
         for (int k = lane; k < J.Kpad; k += 32) {
-            const int e = (int)(((unsigned long long)__double_as_longlong(t[warp][k]) >> 52) & 0x7ff);
+            int e = (int)(((unsigned long long)__double_as_longlong(t[warp][k]) >> 52) & 0x7ff);
+            if constexpr (kScaled) {
+                bad |= e == 0x7ff;
+                if (e != 0) e += kExpBias + sk[k];
+            }
             emax = e > emax ? e : emax;
         }
         emax = __reduce_max_sync(0xffffffffu, emax);
+        if constexpr (kScaled) {
+            bad = __any_sync(0xffffffffu, bad);
+        } else {
+            bad = emax == 0x7ff;
+            if (emax != 0) emax += kExpBias;
+        }
         if (lane == 0) {
-            ex[warp] = emax;
-            J.exps[(int64_t)inst * J.exp_stride + r0 + warp] = emax;
+            ex[warp] = emax - kExpBias;  // not read for a zero row
+            J.exps[(int64_t)inst * J.exp_stride + r0 + warp] = bad ? kExpNan : emax;
         }
     }
     __syncthreads();
@@ -236,7 +290,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
     // Eight consecutive k of one row are contiguous (16 bytes) in the core-
     // matrix order [k/8][row/8][row%8][k%8] of a chunk: a thread digits one
     // such group and writes each slice with a single 16-byte store.
-    const float w7[7] = {1.0f, 0x1p-7f, 0x1p-14f, 0x1p-21f, 0x1p-28f, 0x1p-35f, 0x1p-42f};
+    const float w7[9] = {1.0f, 0x1p-7f, 0x1p-14f, 0x1p-21f, 0x1p-28f, 0x1p-35f, 0x1p-42f, 0x1p-49f, 0x1p-56f};
     for (int g = tid; g < kSplitRows * (J.Kpad / 8); g += kSplitThreads) {
         const int rr = g % kSplitRows, k0 = (g / kSplitRows) * 8;
         const int r = r0 + rr;
@@ -247,8 +301,8 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
             int d0[S], d1[S];
-            digits<S>(t[rr][k0 + j], ex[rr], d0);
-            digits<S>(t[rr][k0 + j + 1], ex[rr], d1);
+            digits<S>(t[rr][k0 + j], kScaled ? sk[k0 + j] : 0, ex[rr], d0);
+            digits<S>(t[rr][k0 + j + 1], kScaled ? sk[k0 + j + 1] : 0, ex[rr], d1);
 #pragma unroll
             for (int p = 0; p < S; ++p) {
                 // w_p = d * 2^(-7p) is exact in bf16 (|d| <= 128)
@@ -396,6 +450,16 @@ __device__ __forceinline__ double f32_to_f64(float f) {
     return __hiloint2double((int)hi, (int)lo);
 }
 
+// Integer of magnitude below 2^53 to FP64 by bit operations (exact).
+__device__ __forceinline__ double int_to_f64(long long v) {
+    if (v == 0) return 0.0;
+    const unsigned long long a = (unsigned long long)(v < 0 ? -v : v);
+    const int lz = __clzll((long long)a);
+    const unsigned long long m = (a << lz) >> 11;  // 53 bits, the leading one at bit 52
+    const unsigned long long bits = ((unsigned long long)(1086 - lz) << 52) + (m - (1ull << 52));
+    return __longlong_as_double((long long)(bits | ((unsigned long long)v & 0x8000000000000000ull)));
+}
+
 // r * 2^e on the exponent bits when the result stays normal, else ldexp.
 __device__ __forceinline__ double scale_pow2(double r, int e) {
     const long long bits = __double_as_longlong(r);
@@ -435,12 +499,6 @@ __device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_addr, uint32_t ran
     return raddr;
 }
 
-__device__ __forceinline__ float ld_dsmem(uint32_t raddr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(raddr) : "memory");
-    return v;
-}
-
 template <int S, int BN>
 struct TcSmem {
     static constexpr int kA = S * TC_BM * TC_BK * 2;   // bytes of A slices per stage
@@ -448,12 +506,11 @@ struct TcSmem {
     static constexpr int kStage = kA + kB;
     static constexpr int kBudget = 225 * 1024;
     static constexpr int kStages = (kBudget / kStage) > 4 ? 4 : (kBudget / kStage);
-    static constexpr int kNacc = S < 6 ? S : 6;
-    // the epilogue stages the FP64 tile (row stride BN + 1) in the idle
-    // stage memory; a K-split CTA keeps its FP32 level accumulators there
-    // too and stages only its (at most half of the) rows
+    // the epilogue stages the FP64 tile (row stride BN + 1) in the idle stage
+    // memory; a K-split CTA parks its folded sums there (FP32 pairs, or 16
+    // bytes of integers for the exact form)
     static constexpr int kOut = TC_BM * (BN + 1) * 8;
-    static constexpr int kRed = kNacc * TC_BM * BN * 4 + (TC_BM / 2) * (BN + 1) * 8;
+    static constexpr int kRed = S > 7 ? TC_BM * (BN + 1) * 16 : TC_BM * (BN + 2) * 8;
     static_assert(kOut <= kStages * kStage, "staging fits the stage memory");
     static constexpr int kData = kStages * kStage > kRed ? kStages * kStage : kRed;
     static constexpr int kExOff = kData + 256;  // staged row / column exponents
@@ -502,7 +559,8 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     if (P.lower_only && n0 >= m0 + TC_BM) return;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int NACC = S < 6 ? S : 6;
+    constexpr bool kExact = S > 7;
+    constexpr int NACC = S < 6 ? S : kExact ? 7 : 6;
     constexpr int kUsed = NACC * BN;
     constexpr int kCols = kUsed <= 32 ? 32 : kUsed <= 64 ? 64 : kUsed <= 128 ? 128 : kUsed <= 256 ? 256 : 512;
     static_assert(kUsed <= 512, "TMEM columns");
@@ -640,11 +698,36 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     // exponent 2047: its digits carry no value) makes the element NaN, as
     // the FP64 product would; a zero row or column otherwise gives 0
     auto finish = [&](float hi, float lo, int eAm, int eBn) -> double {
-        if (eAm == 0x7ff || eBn == 0x7ff) return __longlong_as_double(0x7ff8000000000000ll);
+        if (eAm == kExpNan || eBn == kExpNan) return __longlong_as_double(0x7ff8000000000000ll);
         if (eAm == 0 || eBn == 0) return 0.0;
-        return scale_pow2(f32_to_f64(hi) + f32_to_f64(lo), eAm + eBn - 2058);
+        return scale_pow2(f32_to_f64(hi) + f32_to_f64(lo), eAm + eBn - 2058 - 2 * kExpBias);
+    };
+    // Exact form: the level sums as integers in units of 2^-45 -- level 0, up to
+    // 2^24 2^45, apart from the others, whose sum stays below 2^62 -- so that
+    // adding levels and the CTAs of a K split rounds nothing (levels 6 to 8 share
+    // an accumulator, rounded to a unit); one FMA at the end rounds to FP64.
+    auto fold = [&](const float (&vv)[NACC], int& i0, long long& t) {
+        i0 = __float2int_rn(vv[0]);
+        t = 0;
+        if constexpr (kExact) {
+#pragma unroll
+            for (int l = 1; l < 6; ++l) t += (long long)__float2int_rn(vv[l] * (float)(1ll << (7 * l))) << (45 - 7 * l);
+            t += (long long)__float2int_rn(vv[6] * 0x1p45f);
+        }
+    };
+    auto finish_exact = [&](int i0, long long t, int eAm, int eBn) -> double {
+        if (eAm == kExpNan || eBn == kExpNan) return __longlong_as_double(0x7ff8000000000000ll);
+        if (eAm == 0 || eBn == 0) return 0.0;
+        const long long hi = (long long)i0 + (t >> 45), lo = t & ((1ll << 45) - 1);
+        return scale_pow2(fma(int_to_f64(hi), 0x1p45, int_to_f64(lo)), eAm + eBn - 2058 - 45 - 2 * kExpBias);
     };
     auto combine = [&](const float (&vv)[NACC], int eAm, int eBn) -> double {
+        if constexpr (kExact) {
+            int i0;
+            long long t;
+            fold(vv, i0, t);
+            return finish_exact(i0, t, eAm, eBn);
+        }
         float hi = vv[0], lo = 0.f;
 #pragma unroll
         for (int l = 1; l < NACC; ++l) add2(hi, lo, vv[l]);
@@ -674,6 +757,65 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         // CTAs through distributed shared memory, two elements per 16-byte
         // load, every load of a group in flight together, and writes them
         // out, consecutive threads on consecutive column pairs.
+        if constexpr (kExact) {
+            // the same with integers: {level 0, the others} in 16 bytes
+            constexpr int LDX = BN + 1;
+            int4* RX = (int4*)smem;
+            if (all_ok) {
+                const int q4 = warp & 3, half = warp >> 2;
+                const int row = q4 * 32 + lane;
+#pragma unroll 1
+                for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
+                    float v[NACC][16];
+                    if (nkb > 0) {
+                        tmem_levels16<NACC, BN>(tmem + ((uint32_t)(q4 * 32) << 16) + c0, v);
+                    } else {
+#pragma unroll
+                        for (int l = 0; l < NACC; ++l)
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) v[l][i] = 0.f;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float vv[NACC];
+#pragma unroll
+                        for (int l = 0; l < NACC; ++l) vv[l] = v[l][i];
+                        int i0;
+                        long long t;
+                        fold(vv, i0, t);
+                        RX[row * LDX + c0 + i] = make_int4(i0, 0, (int)t, (int)(t >> 32));
+                    }
+                }
+            }
+            cluster_sync_all();
+            const int nq = (TC_BM + ks - 1) / ks;
+            const int r_lo = (int)rank * nq;
+            const int nr = (r_lo + nq <= TC_BM ? nq : TC_BM - r_lo);
+            uint32_t rb[kTcMaxSplit];
+#pragma unroll
+            for (int q = 0; q < kTcMaxSplit; ++q) rb[q] = q < ks ? dsmem_addr(smem_u32(RX), (uint32_t)q) : 0u;
+            if (all_ok) {
+#pragma unroll 2
+                for (int g = tid; g < nr * BN; g += TC_THREADS2) {
+                    const int row = r_lo + g / BN, c = g % BN;
+                    float4 part[kTcMaxSplit];
+#pragma unroll
+                    for (int q = 0; q < kTcMaxSplit; ++q)
+                        part[q] = q < ks ? ld_dsmem4(rb[q] + (uint32_t)((row * LDX + c) * 16))
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                    int i0 = 0;
+                    long long t = 0;
+#pragma unroll
+                    for (int q = 0; q < kTcMaxSplit; ++q) {
+                        i0 += __float_as_int(part[q].x);
+                        t += (long long)(((unsigned long long)__float_as_uint(part[q].w) << 32) |
+                                         __float_as_uint(part[q].z));
+                    }
+                    store(row, c, finish_exact(i0, t, eAs[row], eBs[c]));
+                }
+            }
+            cluster_sync_all();
+        } else {
         constexpr int LD2 = BN + 2;
         float2* R2 = (float2*)smem;
         if (all_ok) {
@@ -738,6 +880,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
             }
         }
         cluster_sync_all();  // peers are done reading this CTA's accumulators
+        }
     } else {
         // the whole K here: TMEM -> FP64 tile in shared memory -> coalesced writes
         double* Ds = (double*)smem;
@@ -775,6 +918,9 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
             }
         }
     }
+    // a wait gave up: this CTA's part of the tile is marked
+    if (!all_ok)
+        for (int e = tid; e < TC_BM * BN; e += TC_THREADS2) store(e / BN, e % BN, __longlong_as_double(0x7ff8000000000000ll));
     if (!all_ok && tid == 0) {
         // drain (bounded by the fixed limit, not the pipeline's): the final
         // commit, then the last round of bulk copies issued into each stage
@@ -852,7 +998,8 @@ cudaError_t tc_prepare() {
     for (cudaError_t x : {set_smem_attr<3, 64>(), set_smem_attr<4, 64>(), set_smem_attr<5, 64>(),
                           set_smem_attr<6, 64>(), set_smem_attr<7, 64>(), set_smem_attr<3, 32>(),
                           set_smem_attr<4, 32>(), set_smem_attr<5, 32>(), set_smem_attr<6, 32>(),
-                          set_smem_attr<7, 32>()})
+                          set_smem_attr<7, 32>(), set_smem_attr<kExactSlices, 64>(),
+                          set_smem_attr<kExactSlices, 32>()})
         if (x != cudaSuccess) return x;
     g_attr_done[dev] = true;
     return cudaSuccess;
@@ -877,7 +1024,7 @@ size_t tc_workspace_bytes(const GemmProb<double>* probs, int np, int S) {
 cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_bytes, int32_t* err,
                     cudaStream_t s) {
     if (np > kMaxTcProbs) return cudaErrorInvalidValue;
-    if (S != 3 && S != 4 && S != 5 && S != 6 && S != 7) return cudaErrorInvalidValue;
+    if ((S < 3 || S > 7) && S != kExactSlices) return cudaErrorInvalidValue;
     for (int i = 0; i < np; ++i)
         if (probs[i].nterms > 2) return cudaErrorInvalidValue;  // two sources per split job
     SplitLaunch SL;
@@ -961,6 +1108,14 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
             sb.stride = tm.strideB;
             sb.K = tm.K;
             sb.koff = koff;
+            if (S > 7 && tm.ksmode != KS_NONE) {
+                sa.ks = sb.ks = tm.ks;
+                sa.ldks = sb.ldks = tm.ldks;
+                sa.ks_stride = sb.ks_stride = tm.strideKs;
+                sa.kshift = sb.kshift = tm.ksmode == KS_SPD_DIAG ? 1 : 0;
+                sa.ksign = tm.ksmode == KS_SPD_DIAG ? -1 : 1;
+                sb.ksign = -sa.ksign;
+            }
             koff += (int32_t)(ceil_div(tm.K, TC_BK) * TC_BK);
         }
         ja.out = As;
@@ -1029,7 +1184,8 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
             case 4: e = launch_split<4>(SL, (int)split_ctas, s); break;
             case 5: e = launch_split<5>(SL, (int)split_ctas, s); break;
             case 6: e = launch_split<6>(SL, (int)split_ctas, s); break;
-            default: e = launch_split<7>(SL, (int)split_ctas, s); break;
+            case 7: e = launch_split<7>(SL, (int)split_ctas, s); break;
+            default: e = launch_split<kExactSlices>(SL, (int)split_ctas, s); break;
         }
         prof_after(SGB_KCLASS_SPLIT, s, 0.0);
         if (e != cudaSuccess) return e;
@@ -1057,7 +1213,8 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
             case 4: e = launch_tc<4, 64>(TL, (int)gemm_tiles, s); break;
             case 5: e = launch_tc<5, 64>(TL, (int)gemm_tiles, s); break;
             case 6: e = launch_tc<6, 64>(TL, (int)gemm_tiles, s); break;
-            default: e = launch_tc<7, 64>(TL, (int)gemm_tiles, s); break;
+            case 7: e = launch_tc<7, 64>(TL, (int)gemm_tiles, s); break;
+            default: e = launch_tc<kExactSlices, 64>(TL, (int)gemm_tiles, s); break;
         }
     } else {
         switch (S) {
@@ -1065,7 +1222,8 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
             case 4: e = launch_tc<4, 32>(TL, (int)gemm_tiles, s); break;
             case 5: e = launch_tc<5, 32>(TL, (int)gemm_tiles, s); break;
             case 6: e = launch_tc<6, 32>(TL, (int)gemm_tiles, s); break;
-            default: e = launch_tc<7, 32>(TL, (int)gemm_tiles, s); break;
+            case 7: e = launch_tc<7, 32>(TL, (int)gemm_tiles, s); break;
+            default: e = launch_tc<kExactSlices, 32>(TL, (int)gemm_tiles, s); break;
         }
     }
     prof_after(SGB_KCLASS_GEMM_TC, s, fl, issued);

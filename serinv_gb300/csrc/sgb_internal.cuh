@@ -32,7 +32,20 @@ struct GemmTerm {
     int64_t lda, ldb;
     int64_t strideA, strideB;  // element stride between batch instances
     int32_t K;
-    int8_t transA, transB, kmode, _pad;
+    int8_t transA, transB, kmode;
+    // Balance of the contraction index (read by the exact slice products only):
+    // k of op(A) is multiplied and k of op(B) divided by a power of two taken
+    // from the exponent of ks[k * ldks] (batch stride strideKs), so that a
+    // matrix with rows and columns of very different size keeps its digits.
+    int8_t ksmode;  // KS_NONE, KS_SPD_DIAG, KS_TRI_DIAG
+    const T* ks;
+    int64_t ldks, strideKs;
+};
+
+enum KsMode : int8_t {
+    KS_NONE = 0,
+    KS_SPD_DIAG = 1,  // op(A)'s columns grow like the roots of these diagonal entries (of an SPD inverse)
+    KS_TRI_DIAG = 2,  // op(A)'s columns grow like the reciprocals of these diagonal entries (of a factor)
 };
 
 // Cout = alpha * sum_t op(A_t) op(B_t) + beta * op(Cin), over `batch`
@@ -165,6 +178,9 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // SGB_ERR_TIMEOUT if a bounded wait gives up.
 constexpr int kTcBN = 64;
 constexpr int kTcMaxK = 576;
+// Slice count of the products that stand in for FP64 arithmetic: 63 bits below
+// the row maxima, level sums added as integers (sgb_gemm_tc.cu).
+constexpr int kExactSlices = 9;
 size_t tc_workspace_bytes(const GemmProb<double>* probs, int np, int S);
 // Sets the tensor-core kernels' shared-memory attribute on the current
 // device (once); call before capturing launches into a graph.
@@ -180,6 +196,9 @@ cudaError_t bta_symv(const sgb_bta* A, const T* x, int64_t ldx, T* y, int64_t ld
 // x += y over rows x cols.
 template <typename T>
 cudaError_t axpy2d(T* x, int64_t ldx, const T* y, int64_t ldy, int64_t rows, int64_t cols, cudaStream_t s);
+
+// Workspace a native pobtaf runs in without the exact slice products.
+int pobtaf_least_workspace(const sgb_bta* m, size_t* bytes);
 
 // One matrix of a batch plan (sgb_api.cu): its workspace size and the ops.
 size_t plan_item_ws(const sgb_bta* m, int ops, int precision, int64_t nrhs);

@@ -228,6 +228,10 @@ cudaError_t trtri_batched(const T* L, int64_t ldl, int64_t strideL, int64_t m, i
                 w.term[0].strideB = sstride;
                 w.term[0].K = (int32_t)rows2;
                 w.term[0].kmode = KM_LT_M1;
+                w.term[0].ks = L + r1 * ldl + r1;
+                w.term[0].ldks = ldl + 1;
+                w.term[0].strideKs = strideL;
+                w.term[0].ksmode = KS_TRI_DIAG;
                 w.alpha = T(-1);
                 w.Cout = Linv + r1 * ldx + c0;
                 w.ldc = ldx;
