@@ -734,15 +734,18 @@ int pobtaf_run(const sgb_bta* m, int factorize_last_block, int S, int Si, void* 
     SGB_TRY(cudaStreamIsCapturing(s, &cap));
     // one cooperative launch per block (on part of the GPU when captured
     // into a graph beside other work, if the capturing thread allows it);
-    // small blocks, and captures that do not, use the launch-based sweep.
+    // captures that do not, and captured blocks of up to two tiles, use the
+    // launch-based sweep (alone, two tiles take 41 us a block in one launch and
+    // 64 in six: n = 128, b = 64, a = 16 FP64 5.2 ms against 8.3; side by side in
+    // a graph the sweep's small launches leave more of the GPU to the others).
     // In a batch graph the one launch per block also beats the ~25 launches
     // of an FP32 block's tile sweep (measured on the uneven batch: 4.5 %)
     const bool captured = cap != cudaStreamCaptureStatusNone;
     const int pgrid = captured ? capture_panel_grid() : 0;
-    const bool persistent = (!captured || pgrid > 0) && b > 2 * kTile;
+    const bool persistent = !captured || (pgrid > 0 && b > 2 * kTile);
     // 7 slices is the accuracy mode: its TRSMs stay FP64 substitutions (the
     // product with L_ii^{-T} carries kappa(L_ii) times the slice truncation)
-    bool mixed_inverse = S != 0 && (S < 7 || Si != 0) && persistent;
+    bool mixed_inverse = S != 0 && (S < 7 || Si != 0) && persistent && b > 2 * kTile;
     // the launch writes only the upper block triangle of L_ii^{-T}
     // xall (n b x b blocks): keep every L_ii^{-T} for later sweeps on this factor
     if (mixed_inverse) SGB_TRY(cudaMemsetAsync(xall ? xall : Xinv0, 0, sizeof(T) * bb * (xall ? n : 1), s));
@@ -1075,6 +1078,10 @@ int pobtas_native(const sgb_bta* m, T* Bm, int64_t nrhs, int64_t ldb, char trans
     auto Bi = [&](int64_t i) { return Bm + i * b * ldb; };
 
     if (nrhs == 0) return SGB_OK;
+    if (!partial && small_solve_ok<T>(m, nrhs)) {
+        SGB_TRY(small_solve<T>(m, Bm, nrhs, ldb, trans != 'N', s));
+        return SGB_OK;
+    }
     Ctx native;
     // the whole sweep as one launch, which needs the inverses of the diagonal
     // sub-blocks only; the products below take the solves that leave the last
@@ -1843,6 +1850,12 @@ int sgb_pobtaf(const sgb_bta* m, int factorize_last_block, int precision, void* 
     const int Si = parse_inv_slices(precision, S);
     if ((rc = check_ws(workspace, workspace_bytes, taf_bytes(m, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    if (m->dtype == SGB_F64 ? small_factor_ok<double>(m) : small_factor_ok<float>(m)) {
+        int32_t* status = (int32_t*)workspace;
+        SGB_TRY(m->dtype == SGB_F64 ? small_factor<double>(m, factorize_last_block, info, status, s)
+                                    : small_factor<float>(m, factorize_last_block, info, status, s));
+        return SGB_OK;
+    }
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
     SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
     if (m->dtype == SGB_F64)
@@ -1862,6 +1875,12 @@ int sgb_pobtasi(const sgb_bta* m, int invert_last_block, int precision, void* wo
     const int Si = parse_inv_slices(precision, S);
     if ((rc = check_ws(workspace, workspace_bytes, tasi_bytes(m, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    if (m->dtype == SGB_F64 ? small_inverse_ok<double>(m) : small_inverse_ok<float>(m)) {
+        int32_t* status = (int32_t*)workspace;
+        SGB_TRY(m->dtype == SGB_F64 ? small_inverse<double>(m, invert_last_block, status, s)
+                                    : small_inverse<float>(m, invert_last_block, status, s));
+        return SGB_OK;
+    }
     SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
     if (m->dtype == SGB_F64)
         return pobtasi_run<double>(m, invert_last_block, tasi_slices(m, S, workspace_bytes), Si, workspace, s);

@@ -550,12 +550,14 @@ void span(const T* p, int64_t rows, int64_t cols, int64_t ld, int64_t stride, in
     hi = lo + (uintptr_t)(((rows - 1) * ld + cols + (int64_t)(batch - 1) * stride) * (int64_t)sizeof(T));
 }
 
-// The skinny kernel serves a launch when every problem has N <= 8, no
+// The skinny kernel serves a launch when some k is longer than one slab of the
+// small tiles (those wait for memory once: back-sweep at b = 3 22 us a block
+// with this kernel, 7 with theirs) and every problem has N <= 8, no
 // transposed B, no lower-only restriction, and no operand overlapping its
 // output (each CTA reads all of B while others write their rows of C).
 template <typename T>
 bool skinny_ok(const GemmProb<T>* probs, int np) {
-    bool any = false;
+    bool any = false, deep = false;
     for (int i = 0; i < np; ++i) {
         const GemmProb<T>& p = probs[i];
         if (p.M <= 0 || p.N <= 0 || p.batch <= 0) continue;
@@ -566,6 +568,7 @@ bool skinny_ok(const GemmProb<T>* probs, int np) {
         for (int t = 0; t < p.nterms; ++t) {
             const GemmTerm<T>& g = p.term[t];
             if (g.transB) return false;
+            deep = deep || g.K > 64;
             uintptr_t lo, hi;
             span(g.B, g.K, p.N, g.ldb, g.strideB, p.batch, lo, hi);
             if (lo < chi && clo < hi) return false;
@@ -574,7 +577,7 @@ bool skinny_ok(const GemmProb<T>* probs, int np) {
             if (lo < chi && clo < hi) return false;
         }
     }
-    return any;
+    return any && deep;
 }
 
 // Which kernel's tiles a launch gets.

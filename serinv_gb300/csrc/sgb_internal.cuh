@@ -157,6 +157,25 @@ cudaError_t trtri_batched(const T* L, int64_t ldl, int64_t strideL, int64_t m, i
                           T* Linv, int64_t ldx, int64_t strideX, T* scratch, cudaStream_t s,
                           GemmFn<T> fn = nullptr, void* fnctx = nullptr, int64_t sub = 0);
 
+// pobtaf of small blocks in one launch (sgb_small.cu): sets *info to the first
+// bad pivot's row or 0 and *status to 0.
+template <typename T>
+bool small_factor_ok(const sgb_bta* m);
+template <typename T>
+cudaError_t small_factor(const sgb_bta* m, int last, int32_t* info, int32_t* status, cudaStream_t s);
+
+// pobtasi of small blocks in one launch; sets *status to 0.
+template <typename T>
+bool small_inverse_ok(const sgb_bta* m);
+template <typename T>
+cudaError_t small_inverse(const sgb_bta* m, int last, int32_t* status, cudaStream_t s);
+
+// One sweep of pobtas of small blocks in one launch, from the factor alone.
+template <typename T>
+bool small_solve_ok(const sgb_bta* m, int64_t nrhs);
+template <typename T>
+cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, cudaStream_t s);
+
 // Whole-sweep triangular solve in one cluster launch (sgb_solve.cu).  `Li`
 // (n, b, b) holds the inverses of the diagonal sub-blocks of solve_sub() rows
 // of every L_ii at their places (their transposes with li_trans), `Lti` (a, a)

@@ -189,15 +189,19 @@ __device__ __forceinline__ T* row_ptr(const PanelArgs<T>& a, int64_t c1, int64_t
 // (hand-off by value).  With unit >= 0
 // the row is the unit vector e_unit instead of the stored values (a row of
 // the identity, whose solve is a row of L^{-T}); with preset the row starts
-// from y0 (lane = column) instead.  Returns false on a timeout or an error
-// raised elsewhere.
-template <typename T>
+// from y0 (lane = column) instead.  With kApart the products are summed by
+// themselves and taken from the row at once (one more instruction a column):
+// in sequence each rounds at the row's size.  Returns false on a timeout or an
+// error raised elsewhere.
+template <typename T, bool kApart>
 __device__ __forceinline__ bool trsm_row_pipe(T* rp, int w, const T* mt, const T* rv, const unsigned* colcount,
                                               unsigned col_base, int32_t* status, bool sleep, long long spin,
                                               int unit = -1, T* stage_row = nullptr, bool preset = false,
                                               T y0 = T(0)) {
     const int tx = threadIdx.x & 31;
     T y = tx < w ? (unit >= 0 ? T(tx == unit ? 1 : 0) : preset ? y0 : ldcg(rp + tx)) : T(0);
+    const T start = y;
+    T sum = T(0);
     T r = T(0);
     int k = 0;
     long long spins = 0;
@@ -229,7 +233,14 @@ __device__ __forceinline__ bool trsm_row_pipe(T* rp, int w, const T* mt, const T
             for (int u = 0; u < kTile; ++u) {
                 if (u < nb) {
                     const T yk = __shfl_sync(0xffffffffu, y, k + u);
-                    if (tx > k + u) y = fma(-yk, mk[u], y);
+                    if (tx > k + u) {
+                        if constexpr (kApart) {
+                            sum = fma(yk, mk[u], sum);
+                            y = start - sum;
+                        } else {
+                            y = fma(-yk, mk[u], y);
+                        }
+                    }
                 }
             }
             k += nb;
@@ -340,7 +351,8 @@ __device__ __forceinline__ T dot32(const T* a, const T* b, int w) {
     return (a0 + a1) + (a2 + a3);
 }
 
-template <typename T>
+// kApart: a row's updates are summed apart from its elements (see the launch).
+template <typename T, bool kApart>
 __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ PanelArgs<T> a) {
     __shared__ Smem<T> S;
     const int tid = threadIdx.x;
@@ -555,10 +567,12 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
             if (prev && unit < 0) {  // y0 = row(block p) - row(block p-1) * (tile-row p of block p-1)^T
                 const T av = ldcg(rp - kTile + tx);
                 y0 = (fresh || tx >= w) ? T(0) : ldcg(rp + tx);
+                T s = kApart ? T(0) : y0;
 #pragma unroll
-                for (int k = 0; k < kTile; ++k) y0 = fma(-__shfl_sync(0xffffffffu, av, k), tr[tx][k], y0);
+                for (int k = 0; k < kTile; ++k) s = fma(-__shfl_sync(0xffffffffu, av, k), tr[tx][k], s);
+                y0 = kApart ? y0 + s : s;
             }
-            return trsm_row_pipe<T>(rp, w, Mp, rp3, CC, (unsigned)(p * kTile), a.status, true, a.spin, unit, nullptr,
+            return trsm_row_pipe<T, kApart>(rp, w, Mp, rp3, CC, (unsigned)(p * kTile), a.status, true, a.spin, unit, nullptr,
                                     prev && unit < 0, y0);
         };
         if (ty < 4) {
@@ -728,7 +742,7 @@ cudaError_t factor_panel_persistent(T* diag, int64_t m, int64_t ldd, RowSet<T> r
     if (g_panel_grid[dev] == 0) {
         int sms = 0, occ = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_factor_panel<double>, NT, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_factor_panel<double, false>, NT, 0);
         if (e != cudaSuccess) return e;
         int per = occ < 1 ? occ : 1;  // one CTA per SM: cheaper barriers, full FP64 pipe per CTA
         if (per < 1) return cudaErrorLaunchOutOfResources;
@@ -758,7 +772,11 @@ cudaError_t factor_panel_persistent(T* diag, int64_t m, int64_t ldd, RowSet<T> r
     if (e != cudaSuccess) return e;
     void* args[] = {(void*)&a};
     prof_before(s, SGB_KCLASS_PANEL);
-    e = cudaLaunchCooperativeKernel((const void*)k_factor_panel<T>, dim3(G), dim3(NT), args, 0, s);
+    // Two tiles: in FP32 the rows are 1.4e-7 off with updates in sequence and
+    // 6e-8 as sums (n = 128, b = 64), which the tile sweep's products with a tile
+    // inverse also give; longer blocks keep the shorter chain.
+    const void* kernel = m <= 2 * kTile ? (const void*)k_factor_panel<T, true> : (const void*)k_factor_panel<T, false>;
+    e = cudaLaunchCooperativeKernel(kernel, dim3(G), dim3(NT), args, 0, s);
     // useful flops: Cholesky of the m x m block + TRSM of the rows below it
     // (+ the triangular inverse)
     const double md = (double)m;
