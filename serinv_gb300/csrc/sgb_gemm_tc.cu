@@ -26,28 +26,40 @@
 // as integers and rounded once to FP64, and the contraction index balanced by a
 // power of two per k where the caller names a diagonal (GemmTerm::ks): an
 // inverse's columns and the rows they meet may differ by any factor, and a
-// fixed-point row keeps only what lies 63 bits below its largest entry.  One
-// 576 x 512 x 512 launch with 45 slice pairs against 21 at S = 6: 42 us
-// against 31, and its operands' slicing 22 against 16 us.
+// fixed-point row keeps only what lies 63 bits below its largest entry.
 //
 // This is the published Ozaki error-free splitting idea (Ozaki, Ogita,
 // Oishi, Rump) specialised to fixed-point digits and level-grouped exact
 // tensor-core accumulation.
 //
-// Kernel structure (one CTA = one 128 x BN output tile, 6 warps):
+// Kernel structure (one CTA = one 128 x BN output tile, eight warps; a cluster
+// of up to four CTAs shares a tile's K when the tiles leave SMs idle):
 //   * the split kernel writes every slice pre-tiled: one contiguous chunk per
 //     (row tile, 32-wide K block) already in the no-swizzle K-major
 //     core-matrix order (8 rows x 16 bytes per core matrix) that the MMA
-//     descriptors read, so each stage is 2S plain bulk copies;
-//   * warp 4 (producer) streams the chunks with cp.async.bulk into a ring of
-//     2-4 stages, each guarded by a full/empty mbarrier pair;
-//   * warp 5 issues tcgen05.mma (cta_group::1, kind::f16, bf16 inputs, FP32
+//     descriptors read, B's slices side by side within a chunk, so each stage
+//     is S + 1 plain bulk copies; an operand that two problems of a launch
+//     share is sliced once;
+//   * one thread (producer) streams the chunks with cp.async.bulk into a ring
+//     of 2-4 stages, each guarded by a full/empty mbarrier pair;
+//   * one thread issues tcgen05.mma (cta_group::1, kind::f16, bf16 inputs, FP32
 //     accumulation in TMEM) and tcgen05.commit, which frees a stage when its
 //     MMAs have read it;
-//   * warps 0-3 wait for the last commit, read their 32 TMEM lanes with
-//     tcgen05.ld and write FP64;
-//   * every mbarrier wait is bounded; on timeout an error word is set and
-//     the kernel drains (bounded) and frees its TMEM before returning.
+//   * all warps read C_in while the MMAs run, wait for the last commit, read
+//     TMEM with tcgen05.ld, reduce a K split through distributed shared memory
+//     and write FP64;
+//   * every mbarrier wait is bounded; on timeout an error word is set, the
+//     tile is marked NaN and the kernel drains (bounded) and frees its TMEM
+//     before returning.
+//
+// What bounds a product of the sweeps (512 x 512, K = 512, 20 to 32 tiles of
+// ks = 4 CTAs; a thread's time in each part, S = 6): 3.7 us until the slicing
+// launch before it is done, 6.4 us of copies and MMAs, 1.5 us of folding, 4 us
+// of reduction and writing.  One MMA per slice pair, C_in read element by
+// element after the reduction and a releasing barrier at the end (which waits
+// for the stores) took 25.4 us a launch in the factorization and 37.1 us in
+// the selected inverse at n = b = 512; as it is 21.9 and 31.3 us.  S = 9 has 45
+// slice pairs against 21: 14.3 us of copies and MMAs.
 #include <cuda_bf16.h>
 #include <string.h>
 
@@ -90,12 +102,15 @@ struct SplitSrc {
 struct SplitJob {
     SplitSrc src[2];
     int32_t nsrc;
-    __nv_bfloat16* out;   // per instance: [S][Rpad/RT][Kpad/32] chunks of RT x 32 (core-matrix order)
+    __nv_bfloat16* out;   // per instance, A: [S][Rpad/RT][Kpad/32] chunks of RT x 32 (core-matrix order)
+                          // [k/8][row/8][8][8]; B: [Rpad/RT][Kpad/32] chunks of S x RT x 32 in the order
+                          // [k/8][slice][row/8][8][8], so that one MMA takes several slices side by side
     int32_t* exps;        // [Rpad] per instance: kExpBias + biased FP64 exponent of the row max, 0 for a zero
                           // row, kExpNan for a row that holds an Inf or NaN
     int64_t out_stride, exp_stride;
     int32_t R, Rpad, Kpad;
     int32_t RT;           // rows per chunk: 128 for A, the tile width for B
+    int32_t side;         // slices side by side (B)
     int32_t batch;
     int32_t strips, strip_begin;  // kSplitRows-row strips per instance; first CTA of the job
 };
@@ -285,8 +300,9 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
     }
     __syncthreads();
     __nv_bfloat16* out = J.out + (int64_t)inst * J.out_stride;
-    const int64_t slice = (int64_t)J.Rpad * J.Kpad;
     const int nkb = J.Kpad / 32, RT = J.RT;
+    const int sd = J.side ? S : 1;  // slices within a chunk, elements from one slice to the next
+    const int64_t slice = J.side ? (int64_t)RT * 8 : (int64_t)J.Rpad * J.Kpad;
     // Eight consecutive k of one row are contiguous (16 bytes) in the core-
     // matrix order [k/8][row/8][row%8][k%8] of a chunk: a thread digits one
     // such group and writes each slice with a single 16-byte store.
@@ -295,7 +311,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
         const int rr = g % kSplitRows, k0 = (g / kSplitRows) * 8;
         const int r = r0 + rr;
         const int rt = r / RT, ri = r % RT, kb = k0 >> 5, kk = k0 & 31;
-        const int64_t o = ((int64_t)rt * nkb + kb) * (RT * 32) + ((kk >> 3) * (RT >> 3) + (ri >> 3)) * 64 +
+        const int64_t o = ((int64_t)rt * nkb + kb) * (sd * RT * 32) + ((kk >> 3) * sd * (RT >> 3) + (ri >> 3)) * 64 +
                           (ri & 7) * 8;
         uint32_t packed[S][4];
 #pragma unroll
@@ -492,6 +508,12 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// A cluster barrier without memory ordering: the CTAs' last remote reads are done
+// (their values have been used), and the stores after them need not be waited for.
+__device__ __forceinline__ void cluster_sync_reads() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
 // Address of `local_addr` in the shared memory of CTA `rank` of this cluster.
 __device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_addr, uint32_t rank) {
     uint32_t raddr;
@@ -594,9 +616,9 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     // chunk bases: A chunk (p, mt, kb) and B chunk (q, ntile, kb)
     const unsigned char* Ag = (const unsigned char*)(P.A + (int64_t)inst * P.strideA);
     const unsigned char* Bg = (const unsigned char*)(P.B + (int64_t)inst * P.strideB);
-    const int64_t a_slice = (int64_t)P.Mpad * P.Kpad * 2, b_slice = (int64_t)P.Npad * P.Kpad * 2;
+    const int64_t a_slice = (int64_t)P.Mpad * P.Kpad * 2;
     const int64_t a_tile = ((int64_t)mt * nkb_all + kb0) * (TC_BM * TC_BK * 2);
-    const int64_t b_tile = ((int64_t)ntile * nkb_all + kb0) * (BN * TC_BK * 2);
+    const int64_t b_tile = ((int64_t)ntile * nkb_all + kb0) * SM::kB;
 
     if (warp == 4) {
         // producer
@@ -612,21 +634,27 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                 const uint32_t fb = smem_u32(&full[st]);
                 mbar_expect_tx(fb, (uint32_t)SM::kStage);
                 const uint32_t sA = sbase + st * SM::kStage, sB = sA + SM::kA;
+                bulk_g2s(sB, Bg + b_tile + (int64_t)kb * SM::kB, SM::kB, fb);
 #pragma unroll 1
-                for (int p = 0; p < S; ++p) {
+                for (int p = 0; p < S; ++p)
                     bulk_g2s(sA + p * (TC_BM * TC_BK * 2), Ag + p * a_slice + a_tile + (int64_t)kb * (TC_BM * TC_BK * 2),
                              TC_BM * TC_BK * 2, fb);
-                    bulk_g2s(sB + p * (BN * TC_BK * 2), Bg + p * b_slice + b_tile + (int64_t)kb * (BN * TC_BK * 2),
-                             BN * TC_BK * 2, fb);
-                }
             }
             flags[1] = issued;
         }
     } else if (warp == 5) {
         // MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(TC_BM, BN);
-            uint32_t inited = 0;
+            // Slice p of A meets slices q = 0 .. S-1-p of B.  Their levels p + q are
+            // neighbours in TMEM and B's slices neighbours along N in shared memory,
+            // so one MMA of up to 256 columns takes up to 256 / BN of them and A is
+            // read from shared memory once for all (S = 6, BN = 64: 8 MMAs and 74 KB
+            // a 16-wide K step where one MMA a pair took 21 and 126 KB, at 128 bytes
+            // a cycle more than the MMAs themselves need).  Levels past the last
+            // accumulator's are added there one by one.  The first A slice writes
+            // every accumulator, so it alone starts from zero.
+            constexpr int kMaxQ = 256 / BN;
+            constexpr uint32_t kGroup = S * (BN / 8) * 128;  // bytes from one 8-wide K group of B to the next
             for (int kb = 0; kb < nkb; ++kb) {
                 const int st = kb % NS, round = kb / NS;
                 if (!mbar_wait(smem_u32(&full[st]), (uint32_t)(round & 1), L.spin) || flags[0]) {
@@ -641,13 +669,18 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                     for (int p = 0; p < S; ++p) {
                         const uint64_t ad = make_desc(sA + p * (TC_BM * TC_BK * 2) + ks * 2 * (TC_BM / 8) * 128,
                                                       (TC_BM / 8) * 128, 128);
+                        const uint32_t acc = (kb > 0 || ks > 0 || p > 0) ? 1u : 0u;
 #pragma unroll
-                        for (int q = 0; q + p < S; ++q) {
+                        for (int q = 0; q + p < S;) {
+                            const int run = (p + q) >= NACC - 1 ? 1
+                                            : (S - p - q < NACC - p - q ? S - p - q : NACC - p - q) < kMaxQ
+                                                ? (S - p - q < NACC - p - q ? S - p - q : NACC - p - q)
+                                                : kMaxQ;
                             const int l = (p + q) < NACC ? (p + q) : NACC - 1;
-                            const uint64_t bd = make_desc(sB + q * (BN * TC_BK * 2) + ks * 2 * (BN / 8) * 128,
-                                                          (BN / 8) * 128, 128);
-                            tc_mma(tmem + l * BN, ad, bd, idesc, (inited >> l) & 1u);
-                            inited |= 1u << l;
+                            const uint64_t bd = make_desc(sB + ks * 2 * kGroup + q * (BN / 8) * 128, kGroup, 128);
+                            // (past the last level of p = 0 the accumulator holds a value already)
+                            tc_mma(tmem + l * BN, ad, bd, make_idesc(TC_BM, run * BN), (p + q) >= NACC ? 1u : acc);
+                            q += run;
                         }
                     }
                 }
@@ -662,6 +695,28 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     // add, power-of-two scale), staged row-major in shared memory, then
     // written out -- alpha, beta and C_in applied -- with consecutive
     // threads on consecutive columns, so global loads and stores coalesce.
+    // C_in of the elements this thread will write in a K split, while the MMAs run
+    double* C = P.Cout + (int64_t)inst * P.strideC;
+    const double* Ci = P.Cin ? P.Cin + (int64_t)inst * P.strideCin : nullptr;
+    const bool add_c = Ci != nullptr && P.beta != 0.0;
+    auto live = [&](int m, int n) { return m < P.M && n < P.N && !(P.lower_only && n > m); };
+    auto cin = [&](int row, int col) -> double {
+        const int m = m0 + row, n = n0 + col;
+        if (!add_c || !live(m, n)) return 0.0;
+        return P.transCin ? Ci[(int64_t)n * P.ldcin + m] : Ci[(int64_t)m * P.ldcin + n];
+    };
+    constexpr int kOwn = TC_BM / 2 * BN / TC_THREADS2;  // elements a thread writes in a K split, at most
+    double cpre[kOwn];
+    {
+        const int nq = (TC_BM + ks - 1) / ks, r_lo = (int)rank * nq, nr = r_lo + nq <= TC_BM ? nq : TC_BM - r_lo;
+#pragma unroll
+        for (int u = 0; u < kOwn; ++u) {
+            // exact form: single elements; else pairs of neighbours
+            const int g = kExact ? tid + u * TC_THREADS2 : tid + (u / 2) * TC_THREADS2;
+            const int row = kExact ? g / BN : g / (BN / 2), col = kExact ? g % BN : (g % (BN / 2)) * 2 + (u & 1);
+            cpre[u] = ks > 1 && row < nr ? cin(r_lo + row, col) : 0.0;
+        }
+    }
     // every warp reads TMEM in the epilogue: each observes the last commit
     // itself, then orders its tcgen05 loads after it
     bool ok = true;
@@ -669,8 +724,6 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const bool all_ok = !__syncthreads_or(!ok || flags[0] != 0);
     if (!all_ok && tid == 0 && L.err != nullptr) atomicExch(L.err, SGB_ERR_TIMEOUT);
-    double* C = P.Cout + (int64_t)inst * P.strideC;
-    const double* Ci = P.Cin ? P.Cin + (int64_t)inst * P.strideCin : nullptr;
     // the tile's row and column exponents, staged once
     int* eAs = (int*)(smem + SM::kExOff);
     int* eBs = eAs + TC_BM;
@@ -735,16 +788,14 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         return finish(hi, lo, eAm, eBn);
     };
     const bool neg = P.alpha == -1.0, unit = P.alpha == 1.0 || neg;
-    // alpha, beta and C_in applied to one finished element
-    auto store = [&](int row, int col, double r) {
+    // alpha, beta and C_in (read ahead, many at a time, so that its latency is
+    // paid once) applied to one finished element
+    auto store = [&](int row, int col, double r, double cv) {
         const int m = m0 + row, n = n0 + col;
-        if (m >= P.M || n >= P.N || (P.lower_only && n > m)) return;
+        if (!live(m, n)) return;
         if (!unit) r *= P.alpha;
         else if (neg) r = -r;
-        if (Ci != nullptr && P.beta != 0.0) {
-            const double cv = P.transCin ? Ci[(int64_t)n * P.ldcin + m] : Ci[(int64_t)m * P.ldcin + n];
-            r = fma(P.beta, cv, r);
-        }
+        if (add_c) r = fma(P.beta, cv, r);
         C[(int64_t)m * P.ldc + n] = r;
     };
     if (ks > 1) {
@@ -795,26 +846,37 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
 #pragma unroll
             for (int q = 0; q < kTcMaxSplit; ++q) rb[q] = q < ks ? dsmem_addr(smem_u32(RX), (uint32_t)q) : 0u;
             if (all_ok) {
-#pragma unroll 2
-                for (int g = tid; g < nr * BN; g += TC_THREADS2) {
-                    const int row = r_lo + g / BN, c = g % BN;
-                    float4 part[kTcMaxSplit];
 #pragma unroll
-                    for (int q = 0; q < kTcMaxSplit; ++q)
-                        part[q] = q < ks ? ld_dsmem4(rb[q] + (uint32_t)((row * LDX + c) * 16))
-                                         : make_float4(0.f, 0.f, 0.f, 0.f);
-                    int i0 = 0;
-                    long long t = 0;
+                for (int u0 = 0; u0 < kOwn; u0 += 2) {
+                    if (tid + u0 * TC_THREADS2 >= nr * BN) break;
+                    float4 part[2][kTcMaxSplit];
 #pragma unroll
-                    for (int q = 0; q < kTcMaxSplit; ++q) {
-                        i0 += __float_as_int(part[q].x);
-                        t += (long long)(((unsigned long long)__float_as_uint(part[q].w) << 32) |
-                                         __float_as_uint(part[q].z));
+                    for (int h = 0; h < 2; ++h) {
+                        const int g = tid + (u0 + h) * TC_THREADS2;
+                        const int row = g < nr * BN ? r_lo + g / BN : r_lo, c = g % BN;
+#pragma unroll
+                        for (int q = 0; q < kTcMaxSplit; ++q)
+                            part[h][q] = q < ks ? ld_dsmem4(rb[q] + (uint32_t)((row * LDX + c) * 16))
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
-                    store(row, c, finish_exact(i0, t, eAs[row], eBs[c]));
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int g = tid + (u0 + h) * TC_THREADS2;
+                        if (g >= nr * BN) break;
+                        const int row = r_lo + g / BN, c = g % BN;
+                        int i0 = 0;
+                        long long t = 0;
+#pragma unroll
+                        for (int q = 0; q < kTcMaxSplit; ++q) {
+                            i0 += __float_as_int(part[h][q].x);
+                            t += (long long)(((unsigned long long)__float_as_uint(part[h][q].w) << 32) |
+                                             __float_as_uint(part[h][q].z));
+                        }
+                        store(row, c, finish_exact(i0, t, eAs[row], eBs[c]), cpre[u0 + h]);
+                    }
                 }
             }
-            cluster_sync_all();
+            cluster_sync_reads();
         } else {
         constexpr int LD2 = BN + 2;
         float2* R2 = (float2*)smem;
@@ -857,29 +919,40 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         for (int q = 0; q < kTcMaxSplit; ++q) rb[q] = q < ks ? dsmem_addr(smem_u32(R2), (uint32_t)q) : 0u;
         constexpr int G2 = BN / 2;
         if (all_ok) {
-#pragma unroll 1
-            for (int g = tid; g < nr * G2; g += TC_THREADS2) {
-                const int row = r_lo + g / G2, c2 = (g % G2) * 2;
-                float4 part[kTcMaxSplit];
 #pragma unroll
-                for (int q = 0; q < kTcMaxSplit; ++q)
-                    part[q] = q < ks ? ld_dsmem4(rb[q] + (uint32_t)((row * LD2 + c2) * 8))
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-                float h0 = part[0].x, l0 = part[0].y, h1 = part[0].z, l1 = part[0].w;
+            for (int u0 = 0; u0 < kOwn / 2; u0 += 2) {
+                if (tid + u0 * TC_THREADS2 >= nr * G2) break;
+                float4 part[2][kTcMaxSplit];
 #pragma unroll
-                for (int q = 1; q < kTcMaxSplit; ++q) {
-                    add2(h0, l0, part[q].x);
-                    l0 += part[q].y;
-                    add2(h1, l1, part[q].z);
-                    l1 += part[q].w;
+                for (int h = 0; h < 2; ++h) {
+                    const int g = tid + (u0 + h) * TC_THREADS2;
+                    const int row = g < nr * G2 ? r_lo + g / G2 : r_lo, c2 = (g % G2) * 2;
+#pragma unroll
+                    for (int q = 0; q < kTcMaxSplit; ++q)
+                        part[h][q] = q < ks ? ld_dsmem4(rb[q] + (uint32_t)((row * LD2 + c2) * 8))
+                                            : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
-                norm2(h0, l0);
-                norm2(h1, l1);
-                store(row, c2, finish(h0, l0, eAs[row], eBs[c2]));
-                store(row, c2 + 1, finish(h1, l1, eAs[row], eBs[c2 + 1]));
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int g = tid + (u0 + h) * TC_THREADS2;
+                    if (g >= nr * G2) break;
+                    const int row = r_lo + g / G2, c2 = (g % G2) * 2;
+                    float h0 = part[h][0].x, l0 = part[h][0].y, h1 = part[h][0].z, l1 = part[h][0].w;
+#pragma unroll
+                    for (int q = 1; q < kTcMaxSplit; ++q) {
+                        add2(h0, l0, part[h][q].x);
+                        l0 += part[h][q].y;
+                        add2(h1, l1, part[h][q].z);
+                        l1 += part[h][q].w;
+                    }
+                    norm2(h0, l0);
+                    norm2(h1, l1);
+                    store(row, c2, finish(h0, l0, eAs[row], eBs[c2]), cpre[2 * (u0 + h)]);
+                    store(row, c2 + 1, finish(h1, l1, eAs[row], eBs[c2 + 1]), cpre[2 * (u0 + h) + 1]);
+                }
             }
         }
-        cluster_sync_all();  // peers are done reading this CTA's accumulators
+        cluster_sync_reads();  // peers are done reading this CTA's accumulators
         }
     } else {
         // the whole K here: TMEM -> FP64 tile in shared memory -> coalesced writes
@@ -912,15 +985,24 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         __syncthreads();
         if (all_ok) {
 #pragma unroll 1
-            for (int e = tid; e < TC_BM * BN; e += TC_THREADS2) {
-                const int row = e / BN, col = e % BN;
-                store(row, col, Ds[row * (BN + 1) + col]);
+            for (int e0 = tid; e0 < TC_BM * BN; e0 += 8 * TC_THREADS2) {
+                double cv[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int e = e0 + u * TC_THREADS2;
+                    cv[u] = cin(e / BN, e % BN);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int e = e0 + u * TC_THREADS2, row = e / BN, col = e % BN;
+                    store(row, col, Ds[row * (BN + 1) + col], cv[u]);
+                }
             }
         }
     }
     // a wait gave up: this CTA's part of the tile is marked
     if (!all_ok)
-        for (int e = tid; e < TC_BM * BN; e += TC_THREADS2) store(e / BN, e % BN, __longlong_as_double(0x7ff8000000000000ll));
+        for (int e = tid; e < TC_BM * BN; e += TC_THREADS2) store(e / BN, e % BN, __longlong_as_double(0x7ff8000000000000ll), 0.0);
     if (!all_ok && tid == 0) {
         // drain (bounded by the fixed limit, not the pipeline's): the final
         // commit, then the last round of bulk copies issued into each stage
@@ -979,6 +1061,21 @@ cudaError_t launch_split(const SplitLaunch& SL, int ctas, cudaStream_t s) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_split<S>, SL);
+}
+
+// Whether two jobs slice the same numbers into the same layout.
+bool same_operand(const SplitJob& x, const SplitJob& y) {
+    if (x.nsrc != y.nsrc || x.nsrc == 0 || x.R != y.R || x.Rpad != y.Rpad || x.Kpad != y.Kpad || x.RT != y.RT ||
+        x.side != y.side || x.batch != y.batch)
+        return false;
+    for (int q = 0; q < x.nsrc; ++q) {
+        const SplitSrc &a = x.src[q], &b = y.src[q];
+        if (a.X != b.X || a.ld_r != b.ld_r || a.ld_k != b.ld_k || (x.batch > 1 && a.stride != b.stride) || a.K != b.K ||
+            a.koff != b.koff || a.ks != b.ks || a.ldks != b.ldks || (x.batch > 1 && a.ks_stride != b.ks_stride) ||
+            a.ksign != b.ksign || a.kshift != b.kshift)
+            return false;
+    }
+    return true;
 }
 
 std::mutex g_attr_mu;
@@ -1135,10 +1232,22 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         jb.R = p.N;
         jb.Rpad = (int32_t)Npad;
         jb.RT = bn;
+        jb.side = 1;
         jb.Kpad = (int32_t)Kalloc;
         jb.batch = p.batch;
         jb.strips = (int32_t)(Npad / kSplitRows);
+        // an operand that an earlier problem of the launch has too is sliced once
         for (SplitJob* j : {&ja, &jb}) {
+            const SplitJob* same = nullptr;
+            for (int q = 0; q < SL.nj && same == nullptr; ++q)
+                if (same_operand(SL.j[q], *j)) same = &SL.j[q];
+            if (same != nullptr) {
+                j->out = same->out;
+                j->exps = same->exps;
+                j->out_stride = same->out_stride;
+                j->exp_stride = same->exp_stride;
+                continue;
+            }
             if (SL.nj >= kMaxSplitJobs) return cudaErrorInvalidValue;
             j->strip_begin = (int32_t)split_ctas;
             split_ctas += (int64_t)j->strips * j->batch;
@@ -1146,14 +1255,16 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         }
         TcProb tp;
         memset(&tp, 0, sizeof(tp));
-        tp.A = As;
-        tp.B = Bs;
-        tp.eA = eA;
-        tp.eB = eB;
+        tp.A = ja.out;
+        tp.B = jb.out;
+        tp.eA = ja.exps;
+        tp.eB = jb.exps;
         tp.Cin = p.Cin;
         tp.Cout = p.Cout;
-        tp.strideA = tp.strideB = inst_stride_bytes / 2;
-        tp.strideEA = tp.strideEB = inst_stride_bytes / 4;
+        tp.strideA = ja.out_stride;
+        tp.strideB = jb.out_stride;
+        tp.strideEA = ja.exp_stride;
+        tp.strideEB = jb.exp_stride;
         tp.strideCin = p.strideCin;
         tp.strideC = p.strideC;
         tp.ldcin = p.ldcin;
