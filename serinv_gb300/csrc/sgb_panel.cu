@@ -16,8 +16,9 @@
 //   CTAs 1..kNH  helpers: the rows of tile-row p+1 in column block p by
 //                unit-triangular substitution (Y M^T = B, X = Y D^{-1/2}),
 //                following the published columns, handed to each other by
-//                value; then their rows of the update of tile (p+1, p+1),
-//                handed to the factorizer by value; after barrier B they
+//                value as they become final; their rows of the update of
+//                tile (p+1, p+1) follow eight columns behind, handed to
+//                the factorizer by value; after barrier B they
 //                apply column block p to their rows of tile-row p+2 (tiles
 //                (p+2, p+1) and (p+2, p+2)), so nothing the next step needs
 //                waits for the bulk update;
@@ -259,14 +260,14 @@ __device__ __forceinline__ bool trsm_row_pipe(T* rp, int w, const T* mt, const T
 // column, then [32] d) as they land -- no counter, no fence in between.
 // Up to eight columns are polled at once; the leading ones every lane holds
 // are applied.  d^{-1/2} is formed here, lane by lane, as the pivots
-// arrive.  The result also goes to the staging row.  Returns false on a
+// arrive; an element of the result is final once its own column is applied
+// and goes to the row and to the staging row at once.  Returns false on a
 // timeout or an error raised elsewhere.
 template <typename T>
 __device__ __forceinline__ bool trsm_row_vals(T* rp, int w, const T* vc, int32_t* status, T* stage_row,
                                               long long spin) {
     const int tx = threadIdx.x & 31;
     T y = tx < w ? ldcg(rp + tx) : T(0);
-    T r = T(0);
     int k = 0;
     long long rounds = 0;
     while (k < w) {
@@ -306,14 +307,11 @@ __device__ __forceinline__ bool trsm_row_vals(T* rp, int w, const T* vc, int32_t
                 if (!stage_take<T, 1>(dp, want, dv, spin, status)) atomicExch(status, SGB_ERR_TIMEOUT);
                 d = dv[0];
             }
-            r = rsq<T>(d);
+            const T x = y * rsq<T>(d);
+            stage_put(stage_row + tx, x);
+            rp[tx] = x;
         }
         k += navail;
-    }
-    if (tx < w) {
-        const T x = y * r;
-        rp[tx] = x;
-        stage_put(stage_row + tx, x);
     }
     return true;
 }
@@ -448,43 +446,53 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
             // (columns) and p-1 (tile-row), each ordered before tile p's
             // first published columns: acquire those before any poll.
             if (!wait_count(CC, (unsigned)(p * kTile + 1), a.status, &S.flag, a.spin)) return;
+            // Warps 0-3: a row each.  Warps 4-7 follow them: tile-row p+1 by
+            // value, eight columns at a time as all helpers finish them, and
+            // this CTA's rows of the update of tile (p+1, p+1) with those
+            // (one element a thread), so that only the last eight columns'
+            // share is left when the rows end; then by value to the
+            // factorizer.  Taken as a whole after the rows, the update put
+            // 2.0 us between two tiles; following, a tile column of the FP64
+            // form takes 13.5 us instead of 14.0 (mixed factorization at
+            // n = b = 512: 146.1 -> 143.1 ms).
+            bool took = true;
             if (ty < kHelpRows) {
                 const int r = h * kHelpRows + ty;
                 if (r < w2)
                     trsm_row_vals<T>(a.diag + (c1 + r) * a.ldd + c0, w, stV + (p % 3) * kVc, a.status, sL + r * kTile,
                                      a.spin);
-            }
-            // this thread's element of tile (p+1, p+1) (last written by this CTA)
-            const int rr1 = h * kHelpRows + ty, cc1 = tx;
-            const bool own1 = ty < kHelpRows && rr1 < w2 && cc1 <= rr1;
-            const T cold = own1 ? ldcg(a.diag + (c1 + rr1) * a.ldd + c1 + cc1) : T(0);
-            // all of tile-row p+1 by value from the helpers, then their rows
-            // of the update of tile (p+1, p+1), handed to the factorizer by value
-            {
-                constexpr int U = kTile * kTile / NT;
-                const T* sp[U];
-                bool want[U];
-                T v[U];
+            } else {
+                const int gt = tid - 128, rr1 = h * kHelpRows + ty - 4, cc1 = tx;
+                // this thread's element of tile (p+1, p+1) (last written by this CTA)
+                const bool own1 = rr1 < w2 && cc1 <= rr1;
+                const T cold = own1 ? ldcg(a.diag + (c1 + rr1) * a.ldd + c1 + cc1) : T(0);
+                T a0 = T(0), a1 = T(0);
+                for (int k0 = 0; k0 < kTile; k0 += 8) {  // (a CTA without rows there must not wait: the buffer is reset)
+                    const T* sp[2];
+                    bool want[2];
+                    T v[2];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int e = tid + u * NT;
-                    sp[u] = sL + e;
-                    want[u] = e / kTile < w2 && e % kTile < w;
-                }
-                const bool took = stage_take<T, U>(sp, want, v, a.spin, a.status);
+                    for (int u = 0; u < 2; ++u) {
+                        const int r = (gt >> 3) + 16 * u, c = k0 + (gt & 7);
+                        sp[u] = sL + r * kTile + c;
+                        want[u] = took && h * kHelpRows < w2 && r < w2 && c < w;
+                    }
+                    took = stage_take<T, 2>(sp, want, v, a.spin, a.status) && took;
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int e = tid + u * NT;
-                    S.tmp[e / kTile][e % kTile] = want[u] ? v[u] : T(0);
+                    for (int u = 0; u < 2; ++u) S.tmp[(gt >> 3) + 16 * u][k0 + (gt & 7)] = want[u] ? v[u] : T(0);
+                    group_sync(2, 128);
+#pragma unroll
+                    for (int k = k0; k < k0 + 8; k += 2) {
+                        a0 = fma(S.tmp[rr1][k], S.tmp[cc1][k], a0);
+                        a1 = fma(S.tmp[rr1][k + 1], S.tmp[cc1][k + 1], a1);
+                    }
                 }
-                if (__syncthreads_or(!took)) {
-                    if (tid == 0) atomicExch(a.status, SGB_ERR_TIMEOUT);
-                    return;
-                }
+                if (own1 && took) stage_put(stT + ((p + 1) & 1) * kTile * kTile + rr1 * kTile + cc1, cold - (a0 + a1));
             }
-            if (own1)
-                stage_put(stT + ((p + 1) & 1) * kTile * kTile + rr1 * kTile + cc1,
-                          cold - dot32<T>(&S.tmp[rr1][0], &S.tmp[cc1][0], w));
+            if (__syncthreads_or(!took)) {
+                if (tid == 0) atomicExch(a.status, SGB_ERR_TIMEOUT);
+                return;
+            }
             // after the bulk TRSM: column block p applied to their rows of tile-row p+2
             if (!group_barrier(barB, G - 2, epB, a.status, &S.flag, a.spin)) return;
             if (has_next2) {
