@@ -89,6 +89,11 @@ int parse_inv_slices(int precision, int S) {
 // b=224 8787 / 8552, b=240 9441 / 10090, b=512 (n=32) 13522 / 16960.
 constexpr int64_t kExactMinFactor = 240, kExactMinInverse = 224;
 
+// Whether a mixed factorization may take rows * L_ii^{-T} as a product: in place,
+// which only the tensor-core form does (it slices its operands first), and that
+// holds K <= kTcMaxK.
+bool inverse_form(int64_t b) { return b > 2 * kTile && ceil_div(b, 32) * 32 <= kTcMaxK; }
+
 // The slice count of a native FP64 sweep, or 0: the FP64 pipe.
 int exact_slices(const sgb_bta* m, bool inverse) {
     return m->dtype == SGB_F64 && m->b >= (inverse ? kExactMinInverse : kExactMinFactor) &&
@@ -745,7 +750,7 @@ int pobtaf_run(const sgb_bta* m, int factorize_last_block, int S, int Si, void* 
     const bool persistent = !captured || (pgrid > 0 && b > 2 * kTile);
     // 7 slices is the accuracy mode: its TRSMs stay FP64 substitutions (the
     // product with L_ii^{-T} carries kappa(L_ii) times the slice truncation)
-    bool mixed_inverse = S != 0 && (S < 7 || Si != 0) && persistent && b > 2 * kTile;
+    bool mixed_inverse = S != 0 && (S < 7 || Si != 0) && persistent && inverse_form(b);
     // the launch writes only the upper block triangle of L_ii^{-T}
     // xall (n b x b blocks): keep every L_ii^{-T} for later sweeps on this factor
     if (mixed_inverse) SGB_TRY(cudaMemsetAsync(xall ? xall : Xinv0, 0, sizeof(T) * bb * (xall ? n : 1), s));
@@ -1247,7 +1252,7 @@ int pobtaf_permuted_run(const sgb_bta* m, T* buf, int S, int Si, void* ws, int32
     // L_ii^{-T}; the three row sets below become one tensor-core product
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     SGB_TRY(cudaStreamIsCapturing(s, &cap));
-    bool mixed_inverse = S != 0 && (S < 7 || Si != 0) && b > 2 * kTile && cap == cudaStreamCaptureStatusNone;
+    bool mixed_inverse = S != 0 && (S < 7 || Si != 0) && inverse_form(b) && cap == cudaStreamCaptureStatusNone;
     if (mixed_inverse) SGB_TRY(cudaMemsetAsync(Xinv, 0, sizeof(T) * bb, s));
     {   // buf[1] = Lo[0]^T  (pobtaf.py:203)
         GemmProb<T> c = copy_prob<T>(buf + bb, b, Lo, b, b, b);
@@ -1577,7 +1582,7 @@ int pobtas_refine_run(const sgb_bta* A, const sgb_bta* L, T* B, int64_t nrhs, in
 bool item_keeps_inverses(const sgb_bta* m, int precision, int ops) {
     const int S = parse_precision(precision, m->dtype);
     return (ops & SGB_OP_POBTAF) && (ops & (SGB_OP_POBTAS | SGB_OP_POBTASI)) && m->dtype == SGB_F64 && S > 0 &&
-           S < 7 && m->b > 2 * kTile && capture_panel_grid() > 0;
+           S < 7 && inverse_form(m->b) && capture_panel_grid() > 0;
 }
 
 }  // namespace
