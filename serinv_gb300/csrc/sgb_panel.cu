@@ -48,6 +48,8 @@
 // never from a possibly stale L1 line.
 #include <math.h>
 
+#include <type_traits>
+
 #include "sgb_internal.cuh"
 #include "sgb_tile.cuh"
 
@@ -532,18 +534,42 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
         // Then barrier B (with the helpers).  The rows never wait for the
         // bulk update, and the bulk update runs while the rows follow the
         // pivots.
-        const unsigned nwk = G - kW0, wk = cta - kW0;
+        const int nwk = (int)G - kW0, wk = (int)cta - kW0;
         const bool prev = p >= 1;  // the trailing update of step p-1 is due
         const int64_t off0 = w2;
         const int64_t nbase = (m - c1) + a.r1rows + a.r2rows - off0;
         const int64_t nrows = nbase + (a.xinv ? c1 : 0);
         if (tid == 0) S.rowq[(p + 1) & 1] = 0;  // the next step's row counter (used after barrier B)
-        // This CTA's q-th row of the step: wk*4 + (q & 3) + (q / 4) * nwk*4.
-        // Warps 0-3 start with q = ty and take every further q from a shared
+        // Rows go to the CTAs four at a time.  Warps 0-3 start with q = ty and take every further q from a shared
         // counter; when the rows outnumber the first round (the tall panels
         // of the FP64 forms), warps 4-7 join once their share of the update
         // is done, with their own copy of the tile-row operand.
         const bool tall = nrows > (int64_t)nwk * 4;
+        // The update of step q = p-1: column block q, trailing panel from c1q = c0.
+        // D tiles (ti, cj) with ti >= 2 and 1 <= cj <= ti, then the tiles of the
+        // other row sets (the last: tile-rows of L^{-T} not zero in block q)
+        // with cj >= 1.
+        const int64_t c0q = c0 - kTile, c1q = c0;
+        const int ntd = (int)((m - c1q + kTile - 1) / kTile);  // tile-rows from tile-row p
+        const int n1 = (int)((a.r1rows + kTile - 1) / kTile), n2 = (int)((a.r2rows + kTile - 1) / kTile);
+        const int nx = a.xinv ? (int)p : 0;
+        const int tiles_d = ntd >= 2 ? ntd * (ntd - 1) / 2 - 1 : 0;
+        const int total = prev && ntd >= 2 ? tiles_d + (n1 + n2 + nx) * (ntd - 1) : 0;
+        // An FP64 tile keeps a worker's FP64 units (64 cycles a warp
+        // instruction and SM quarter) busy for 8 us, so where halves leave a
+        // shorter last round the workers take half tiles: n=128 b=512 with 390
+        // to 40 tiles a step 51.9 -> 49.9 ms (quarters: 51.9; halves throughout:
+        // the mixed form, 99 to 134 tiles a step, 142.4 -> 143.2 ms).
+        const int rounds = (total + nwk - 1) / nwk, rounds2 = (2 * total + nwk - 1) / nwk;
+        const bool halves = sizeof(T) == 8 && rounds2 < 2 * rounds;
+        const int units = halves ? 2 * total : total;
+        // Where the update is the longer part (three rounds of halves, 12 us
+        // beside a tile's 14 us), the workers without a unit in the last round
+        // take that much more of the rows (eight rows are half a tile's FP64
+        // instructions): 49.9 -> 47.3 ms.
+        const int heavy = sizeof(T) == 8 && rounds2 >= 3 ? units - (halves ? rounds2 - 1 : rounds - 1) * nwk : 0;
+        const int light = nwk - heavy, extra = heavy > 0 ? (halves ? 2 : 4) : 0;  // groups of four rows
+        const int seat = wk >= heavy ? wk - heavy : wk - heavy + nwk;             // the light ones first
         // tile-row p in column block p-1 (the helpers' rows of step p-1),
         // the operand of every row's share of the update: to S.x (warps
         // 0-3) or S.u (warps 4-7)
@@ -553,7 +579,12 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                 dst[r][k] = r < w ? ldcg(a.diag + (c0 + r) * a.ldd + (c0 - kTile) + k) : T(0);
             }
         };
-        auto row_of = [&](int64_t q) { return (int64_t)wk * 4 + (q & 3) + (q >> 2) * (int64_t)nwk * 4; };
+        auto row_of = [&](int64_t q) {  // this CTA's q-th row
+            int64_t g = q >> 2;
+            if (seat < light && g < extra) g = g * light + seat;
+            else g = extra * light + (g - (seat < light ? extra : 0)) * nwk + seat;
+            return g * 4 + (q & 3);
+        };
         auto next_q = [&]() -> int64_t {
             int g = 0;
             if (tx == 0) g = atomicAdd(&S.rowq[p & 1], 1);
@@ -593,15 +624,6 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                 if (r >= nrows || !do_row(r, S.x)) break;
             }
         } else if (prev) {
-            // step q = p-1: column block q, trailing panel from c1q = c0
-            const int64_t c0q = c0 - kTile, c1q = c0;
-            const int64_t ntd = (m - c1q + kTile - 1) / kTile;  // tile-rows from tile-row p
-            const int64_t n1 = (a.r1rows + kTile - 1) / kTile, n2 = (a.r2rows + kTile - 1) / kTile;
-            const int64_t nx = a.xinv ? p : 0;  // tile-rows of L^{-T} not zero in block q
-            // D tiles (ti, cj) with ti >= 2 and 1 <= cj <= ti, then the tiles
-            // of the other row sets with cj >= 1
-            const int64_t tiles_d = ntd >= 2 ? ntd * (ntd - 1) / 2 - 1 : 0;
-            const int64_t total = ntd >= 2 ? tiles_d + (n1 + n2 + nx) * (ntd - 1) : 0;
             const T* Bpan = a.diag + c1q * a.ldd + c0q;
             struct TileRef {
                 T* C;
@@ -609,13 +631,13 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                 int64_t ldc, rows, cols, cj;
                 bool fresh;  // C holds no value yet (L^{-T} tile-row q): C = -update
             };
-            auto tile_ref = [&](int64_t t) {
+            auto tile_ref = [&](int t) {
                 TileRef R;
                 R.fresh = false;
                 int64_t ti;
                 if (t < tiles_d) {  // (ti - 1, cj - 1) over the triangle of ntd - 1 tile-rows, from its second tile
-                    const int64_t tt = t + 1;
-                    int64_t ui = (int64_t)((sqrt(8.0 * (double)tt + 1.0) - 1.0) * 0.5);
+                    const int tt = t + 1;
+                    int ui = (int)((sqrtf(8.0f * (float)tt + 1.0f) - 1.0f) * 0.5f);
                     while (ui * (ui + 1) / 2 > tt) --ui;
                     while ((ui + 1) * (ui + 2) / 2 <= tt) ++ui;
                     ti = ui + 1;
@@ -625,9 +647,9 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                     R.ldc = a.ldd;
                     R.rows = (m - c1q) - ti * kTile;
                 } else {
-                    const int64_t u = t - tiles_d;
-                    const int64_t set = u / (ntd - 1);
-                    R.cj = 1 + u % (ntd - 1);
+                    const int u = t - tiles_d;
+                    const int set = u / (ntd - 1);
+                    R.cj = 1 + (u - set * (ntd - 1));
                     if (set < n1) {
                         ti = set;
                         R.C = a.r1 + ti * kTile * a.r1ld + c1q;
@@ -654,71 +676,95 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                 if (R.cols > kTile) R.cols = kTile;
                 return R;
             };
-            // 128 threads, 8 outputs each: rows cy + 8 i (i < 4), columns cx + 16 j (j < 2)
+            // 128 threads; a unit of 8 NI rows of a tile, outputs of a thread:
+            // rows cy + 8 i (i < NI), columns cx + 16 j (j < 2)
             const int gt = tid - 128, cx = gt & 15, cy = gt >> 4;
-            constexpr int U = kTile * kTile / 128;
-            T va[U], vb[U], vc[4][2];
-            auto fetch = [&](const TileRef& R) {
+            auto sweep = [&](auto ni) {
+                constexpr int NI = decltype(ni)::value;
+                constexpr int kParts = 4 / NI;  // units of a tile
+                constexpr int UA = kTile * kTile / 128 / kParts, UB = kTile * kTile / 128;
+                T va[UA], vb[UB], vc[NI][2];
+                auto unit = [&](int t) {
+                    TileRef R = tile_ref(t / kParts);
+                    const int r0 = (t % kParts) * (8 * NI);
+                    R.A += r0 * R.ldc;
+                    R.C += r0 * R.ldc;
+                    R.rows -= r0;
+                    return R;
+                };
+                auto fetch = [&](const TileRef& R) {
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int e = gt + u * 128, r = e / kTile, k = e % kTile;
-                    va[u] = r < R.rows ? ldcg(R.A + (int64_t)r * R.ldc + k) : T(0);
-                    vb[u] = r < R.cols ? ldcg(Bpan + (R.cj * kTile + r) * a.ldd + k) : T(0);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const int r = cy + 8 * i, c = cx + 16 * j;
-                        vc[i][j] = (!R.fresh && r < R.rows && c < R.cols)
-                                       ? ldcg(R.C + (int64_t)r * R.ldc + R.cj * kTile + c)
-                                       : T(0);
+                    for (int u = 0; u < UA; ++u) {
+                        const int e = gt + u * 128, r = e / kTile, k = e % kTile;
+                        va[u] = r < R.rows ? ldcg(R.A + (int64_t)r * R.ldc + k) : T(0);
                     }
-            };
-            int64_t t = wk;
-            TileRef cur;
-            if (t < total) {
-                cur = tile_ref(t);
-                fetch(cur);
-            }
-            for (; t < total; t += nwk) {
-                group_sync(2, 128);  // the previous tile's operands are no longer read
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int e = gt + u * 128;
-                    S.s[e / kTile][e % kTile] = va[u];
-                    S.tmp[e / kTile][e % kTile] = vb[u];
-                }
-                T acc[4][2];
+                    for (int u = 0; u < UB; ++u) {
+                        const int e = gt + u * 128, r = e / kTile, k = e % kTile;
+                        vb[u] = r < R.cols ? ldcg(Bpan + (R.cj * kTile + r) * a.ldd + k) : T(0);
+                    }
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                    for (int i = 0; i < NI; ++i)
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) acc[i][j] = vc[i][j];
-                group_sync(2, 128);
-                const TileRef now = cur;
-                if (t + nwk < total) {  // next tile's operands in flight during this tile's FMAs
-                    cur = tile_ref(t + nwk);
+                        for (int j = 0; j < 2; ++j) {
+                            const int r = cy + 8 * i, c = cx + 16 * j;
+                            vc[i][j] = (!R.fresh && r < R.rows && c < R.cols)
+                                           ? ldcg(R.C + (int64_t)r * R.ldc + R.cj * kTile + c)
+                                           : T(0);
+                        }
+                };
+                int t = wk;
+                TileRef cur;
+                if (t < units) {
+                    cur = unit(t);
                     fetch(cur);
                 }
-                for (int k = 0; k < kTile; ++k) {
-                    T av[4], bv[2];
+                for (; t < units; t += nwk) {
+                    group_sync(2, 128);  // the previous unit's operands are no longer read
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) av[i] = S.s[cy + 8 * i][k];
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) bv[j] = S.tmp[cx + 16 * j][k];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int j = 0; j < 2; ++j) acc[i][j] = fma(-av[i], bv[j], acc[i][j]);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const int r = cy + 8 * i, c = cx + 16 * j;
-                        if (r < now.rows && c < now.cols) now.C[(int64_t)r * now.ldc + now.cj * kTile + c] = acc[i][j];
+                    for (int u = 0; u < UA; ++u) {
+                        const int e = gt + u * 128;
+                        S.s[e / kTile][e % kTile] = va[u];
                     }
-            }
+#pragma unroll
+                    for (int u = 0; u < UB; ++u) {
+                        const int e = gt + u * 128;
+                        S.tmp[e / kTile][e % kTile] = vb[u];
+                    }
+                    T acc[NI][2];
+#pragma unroll
+                    for (int i = 0; i < NI; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) acc[i][j] = vc[i][j];
+                    group_sync(2, 128);
+                    const TileRef now = cur;
+                    if (t + nwk < units) {  // next unit's operands in flight during this one's FMAs
+                        cur = unit(t + nwk);
+                        fetch(cur);
+                    }
+                    for (int k = 0; k < kTile; ++k) {
+                        T av[NI], bv[2];
+#pragma unroll
+                        for (int i = 0; i < NI; ++i) av[i] = S.s[cy + 8 * i][k];
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) bv[j] = S.tmp[cx + 16 * j][k];
+#pragma unroll
+                        for (int i = 0; i < NI; ++i)
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) acc[i][j] = fma(-av[i], bv[j], acc[i][j]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < NI; ++i)
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            const int r = cy + 8 * i, c = cx + 16 * j;
+                            if (r < now.rows && c < now.cols)
+                                now.C[(int64_t)r * now.ldc + now.cj * kTile + c] = acc[i][j];
+                        }
+                }
+            };
+            if (halves) sweep(std::integral_constant<int, 2>{});
+            else sweep(std::integral_constant<int, 4>{});
         }
         if (ty >= 4 && tall) {  // the update's share done: help with the rows still left
             if (prev) {
