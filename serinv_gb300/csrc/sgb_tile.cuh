@@ -34,16 +34,16 @@ template <>
 __device__ __forceinline__ float rsq<float>(float x) { return rsqrtf(x); }
 
 template <typename T>
-struct Smem {
+struct alignas(16) Smem {
     T s[kTile][kTile + 1];
-    T x[kTile][kTile + 1];
+    T x[kTile][kTile + 1];  // x, tmp, u: 16-byte aligned
     T tmp[kTile][kTile + 1];
     T u[kTile][kTile + 1];
     T yv[kTile];
     unsigned short tri[kTile * (kTile + 1) / 2];  // (row << 8) | col of the lower triangle, row-major
     int fail;
     int flag;
-    int pub;      // factor_tile_m: columns the companion has completed
+    int pub;      // factor_tile_m: columns completed
     int rowq[2];  // column-block kernel workers: row counters of alternate steps
 };
 
@@ -433,11 +433,75 @@ __device__ void factor_tile(Smem<T>& S, T* tile, int64_t ld, int nb, int zero_ri
     __syncthreads();
 }
 
+// Columns 8 w .. 8 w + 7 of an FP32 tile on one warp (lane = row): the columns
+// before them as their warps finish them, then its own, one pivot after another
+// in registers.  An FP32 column has some 20 instructions of arithmetic, and with
+// a warp for the pivots, one for the next column and four for the rest, the two
+// barrier hops of every column took 403 cycles; here a hop lies between two
+// warps' columns only (206 cycles a column).  u = a'_ij (rows below the pivot) and
+// v = - u / d_j of every finished column stand in S.u and S.tmp (32 x 32), v as
+// M(:, j) in S.x as well; S.pub counts the columns.
+__device__ __forceinline__ void tile_columns(Smem<float>& S, int w) {
+    constexpr int W = kTile / 4;
+    const int lane = threadIdx.x & 31, c0 = w * W;
+    float* up = &S.u[0][0];
+    float* vp = &S.tmp[0][0];
+    const unsigned pub = smem_u32(&S.pub);
+    float s[W], dg = S.s[lane][lane];
+#pragma unroll
+    for (int c = 0; c < W; ++c) s[c] = lane > c0 + c ? S.s[lane][c0 + c] : 0.f;
+    int have = 0;
+    for (int j = 0; j < c0; ++j) {
+        // ends: that column's warp finishes it in any case (bounded all the same)
+        for (int i = 0; have <= j && i < (1 << 26); ++i)
+            asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(have) : "r"(pub) : "memory");
+        const float u = up[j * kTile + lane], v = vp[j * kTile + lane];
+        float vb[W];
+#pragma unroll
+        for (int c = 0; c < W; c += 4) {
+            const float4 f = *reinterpret_cast<const float4*>(&vp[j * kTile + c0 + c]);
+            vb[c] = f.x, vb[c + 1] = f.y, vb[c + 2] = f.z, vb[c + 3] = f.w;
+        }
+        dg = fmaf(u, v, dg);
+#pragma unroll
+        for (int c = 0; c < W; ++c) s[c] = fmaf(u, vb[c], s[c]);
+    }
+    float d = __shfl_sync(0xffffffffu, dg, c0);
+    int fail = kTile + 1;
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+        const int j = c0 + c;
+        const bool ok = pivot_ok(d);
+        Rcp<float> r;
+        r.first(d);
+        float inv = r.second();
+        if (!Rcp<float>::plain(d)) inv = ok ? 1.0f / d : NAN;
+        const float u = lane > j ? s[c] : 0.f, v = -(u * inv);
+        dg = fmaf(u, v, dg);
+        const float next = c + 1 < W ? __shfl_sync(0xffffffffu, dg, j + 1) : 0.f;
+        up[j * kTile + lane] = u;
+        vp[j * kTile + lane] = v;
+        S.x[lane][j] = 0.f - v;
+        if (lane == 0) S.yv[j] = d;
+        float vk[W];
+#pragma unroll
+        for (int k = c + 1; k < W; ++k) vk[k] = __shfl_sync(0xffffffffu, v, c0 + k);
+        __syncwarp();
+        if (lane == 0) asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(pub), "r"(j + 1) : "memory");
+#pragma unroll
+        for (int k = c + 1; k < W; ++k) s[k] = fmaf(u, vk[k], s[k]);
+        fail = !ok && fail > kTile ? j + 1 : fail;
+        d = next;
+    }
+    if (lane == 0 && fail <= kTile) atomicMin(&S.fail, fail);
+}
+
 // The pipeline part of factor_tile alone, for the persistent column-block
 // kernel: after it, S.x holds the strict lower part of M (zero elsewhere)
 // and S.yv the pivots d (1 beyond nb), so L = M diag(d)^{1/2}; no inverse,
-// no output.  The sequential chain is split between two warps on different
-// SM quarters so that each carries as few FP64 instructions as possible:
+// no output.  FP32 tiles: warps 0-3 take eight columns each (tile_columns).
+// FP64: the sequential chain is split between two warps on different SM
+// quarters so that each carries as few FP64 instructions as possible:
 //
 // * warp 0 (pivot) keeps only the pivots: from 1/d_j and the pair
 //   (q_{j+1}, e_{j+1}) = (a'_{j+1,j}^2, diagonal of column j+1 through
@@ -512,13 +576,18 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
         if (c < r) S.tri[r * (r - 1) / 2 + c] = (unsigned short)((r << 8) | c);  // strict lower, row-major
     }
     if (tid < kTile) S.yv[tid] = T(1);
+    constexpr bool kRegs = sizeof(T) == 4;
     if (tid == 0) {
-        S.fail = 0;
+        S.fail = kRegs ? kTile + 1 : 0;
         S.pub = 0;
     }
     if (timed_out && status != nullptr) atomicExch(status, SGB_ERR_TIMEOUT);
     __syncthreads();
-    if (warp == 0) {
+    if (kRegs && warp < 4) {
+        // (columns from nb on are those of the identity)
+        if constexpr (kRegs)
+            if (warp * (kTile / 4) < nb) tile_columns(S, warp);
+    } else if (warp == 0) {
         T d = S.s[0][0];
         bool ok = pivot_ok(d);
         T inv = ok ? rcp_pivot(d) : T(NAN);
@@ -585,6 +654,7 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
                     if (avail > done || ++spins > (1ll << 26)) break;
                 }
                 if (avail <= done) break;  // the waits of the consumers time out and report it
+                avail = avail < nb ? avail : nb;
                 for (int k = done; k < avail; ++k) mt[k * kTile + lane] = S.x[lane][k];
                 if (lane >= done && lane < avail) {
                     const T d = S.yv[lane];
@@ -616,12 +686,13 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
                     if (avail > done || ++spins > (1ll << 26)) break;
                 }
                 if (avail <= done) break;
+                avail = avail < nb ? avail : nb;
                 if (lane >= done && lane < avail) stage_put(vcols + kTile * kTile + lane, S.yv[lane]);
                 for (int k = done; k < avail; ++k) stage_put(vcols + k * kTile + lane, S.x[lane][k]);
                 done = avail;
             }
         }
-    } else {
+    } else if (!kRegs) {
         const int wid = (warp < 4 ? warp - 2 : warp - 4) * 32 + lane;  // 0..127
         for (int k = 0; k < nb; ++k) {
             nbar_sync(1 + (k & 1), kCons);  // READY(k)
@@ -636,7 +707,7 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
         }
     }
     __syncthreads();
-    if (tid == 0 && S.fail != 0 && info != nullptr) atomicCAS(info, 0, (int32_t)(row0 + S.fail));
+    if (tid == 0 && S.fail != (kRegs ? kTile + 1 : 0) && info != nullptr) atomicCAS(info, 0, (int32_t)(row0 + S.fail));
 }
 
 // The tile's L = M diag(d)^{1/2} from M (strict lower, in m), the pivots d

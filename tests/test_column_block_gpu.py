@@ -24,3 +24,28 @@ def test_update_rounds(b, a, dtype, precision, tol):
     oracle.pobtaf(*ref)
     for x, y in zip(d, ref):
         assert np.linalg.norm(x.cpu().numpy() - y) <= tol * max(np.linalg.norm(y), 1e-300)
+
+
+# FP32 diagonal tiles: eight columns a warp, the last tile of every width
+@pytest.mark.parametrize("b", [65, 71, 72, 73, 95, 98, 127])
+def test_fp32_tile_widths(b):
+    m = generate(3, b, 9, 1, seed=b, dtype=np.float32)
+    d = [torch.from_numpy(x.copy()).cuda() for x in m.arrays()]
+    ref = [x.astype(np.float64) for x in m.arrays()]
+    sg.pobtaf(*d)
+    oracle.pobtaf(*ref)
+    for x, y in zip(d, ref):
+        assert np.linalg.norm(x.cpu().numpy() - y) <= 1e-5 * max(np.linalg.norm(y), 1e-300)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("bad", [(0,), (7,), (8, 9), (31,), (32, 70), (47, 33), (70,)])
+def test_first_bad_pivot(bad, dtype):
+    b = 71
+    D = np.repeat(4 * np.eye(b, dtype=dtype)[None], 3, 0)
+    D[:, 1:, :-1] += np.eye(b - 1, dtype=dtype)
+    for k in bad:
+        D[1, k, k] = -1 if k != 33 else np.nan
+    d = [torch.from_numpy(x).cuda() for x in (D, np.zeros((2, b, b), dtype))]
+    with pytest.raises(np.linalg.LinAlgError, match=f"^{b + min(bad) + 1}-th"):
+        sg.pobtf(*d)
