@@ -11,17 +11,18 @@
 //   CTA 0        factorizer: diagonal tile p as L = M D^{1/2} (the pivot
 //                pipeline of factor_tile_m), whose warp 4 publishes the
 //                columns of M, d and d^{-1/2} as they are produced
-//                (counter of published columns), then counter F at the end
-//                of the tile; tile p+1 arrives by value from the helpers;
+//                (counter of published columns); tile p+1 arrives by
+//                value from the helpers;
 //   CTAs 1..kNH  helpers: the rows of tile-row p+1 in column block p by
 //                unit-triangular substitution (Y M^T = B, X = Y D^{-1/2}),
 //                following the published columns, handed to each other by
 //                value as they become final; their rows of the update of
 //                tile (p+1, p+1) follow eight columns behind, handed to
 //                the factorizer by value; after barrier B they
-//                apply column block p to their rows of tile-row p+2 (tiles
-//                (p+2, p+1) and (p+2, p+2)), so nothing the next step needs
-//                waits for the bulk update;
+//                apply column block p to their rows of tile-row p+2: to
+//                tile (p+2, p+1) at once, kept in shared memory for the
+//                next step's rows, to tile (p+2, p+2) during them, so
+//                nothing the next step needs waits for the bulk update;
 //   CTA kNH+1    L writer: from M_p, d_p the tile's L into the matrix
 //                (counter I);
 //   CTAs kNH+2.. workers: warps 0-3 the other rows below tile p (and, with
@@ -78,7 +79,7 @@ struct PanelArgs {
                  // [3][32 * 32 + 32] staged columns of M and d
     int32_t* info;
     int64_t row0;
-    unsigned* bar;    // [0] F, [1] I, [4] barrier B, [8] columns of M
+    unsigned* bar;    // [1] I, [4] barrier B, [8] columns of M
                       // published; zero at launch
     int32_t* status;  // SGB_ERR_TIMEOUT on a stuck wait
     long long spin;   // poll limit of every bounded wait
@@ -143,14 +144,6 @@ __device__ __forceinline__ bool wait_count(const unsigned* ctr, unsigned target,
         }
         *sflag = ok;
     }
-    __syncthreads();
-    return *sflag != 0;
-}
-
-// CTA-uniform check of the status word (also a CTA barrier).
-__device__ __forceinline__ bool cta_ok(const int32_t* status, int* sflag) {
-    __syncthreads();
-    if (threadIdx.x == 0) *sflag = !status_bad(status);
     __syncthreads();
     return *sflag != 0;
 }
@@ -262,33 +255,39 @@ __device__ __forceinline__ bool trsm_row_pipe(T* rp, int w, const T* mt, const T
 // column, then [32] d) as they land -- no counter, no fence in between.
 // Up to eight columns are polled at once; the leading ones every lane holds
 // are applied.  d^{-1/2} is formed here, lane by lane, as the pivots
-// arrive; an element of the result is final once its own column is applied
-// and goes to the row and to the staging row at once.  Returns false on a
-// timeout or an error raised elsewhere.
+// arrive; an element of the result is final once its own column is applied,
+// and goes to the row and to the staging row with the others of its eight
+// columns (a square root takes the warp 500 cycles, for one lane or all).  y:
+// this lane's element of the row.  Returns false on a timeout or an error raised elsewhere.
 template <typename T>
-__device__ __forceinline__ bool trsm_row_vals(T* rp, int w, const T* vc, int32_t* status, T* stage_row,
+__device__ __forceinline__ bool trsm_row_vals(T* rp, T y, int w, const T* vc, int32_t* status, T* stage_row,
                                               long long spin) {
     const int tx = threadIdx.x & 31;
-    T y = tx < w ? ldcg(rp + tx) : T(0);
+    T d = T(1);
     int k = 0;
     long long rounds = 0;
-    while (k < w) {
-        const int nb = (w - k) < 8 ? (w - k) : 8;
-        decltype(Staged<T>::ld(vc)) raw[8];
+    decltype(Staged<T>::ld(vc)) raw[8], rd;
+    // columns k .. and this lane's pivot if it is among them (staged before its
+    // column; polled below only if it has not landed yet), up to the next
+    // multiple of eight
+    auto fetch = [&]() {
+        const int nb = (w - k) < 8 - (k & 7) ? (w - k) : 8 - (k & 7);
 #pragma unroll
         for (int u = 0; u < 8; ++u) raw[u] = u < nb ? Staged<T>::ld(vc + (k + u) * kTile + tx) : Staged<T>::kSentinel;
-        // this lane's pivot in the same round (staged before its column;
-        // polled below only if it has not landed yet)
-        const auto rd = (tx >= k && tx < k + nb) ? Staged<T>::ld(vc + kTile * kTile + tx) : Staged<T>::kSentinel;
+        rd = (tx >= k && tx < k + nb) ? Staged<T>::ld(vc + kTile * kTile + tx) : Staged<T>::kSentinel;
+    };
+    fetch();
+    while (k < w) {
         int navail = 0;
 #pragma unroll
         for (int u = 0; u < 8; ++u)
-            if (navail == u && u < nb && __all_sync(0xffffffffu, raw[u] != Staged<T>::kSentinel)) navail = u + 1;
+            if (navail == u && __all_sync(0xffffffffu, raw[u] != Staged<T>::kSentinel)) navail = u + 1;
         if (navail == 0) {
             if (++rounds > spin || ((rounds & 63) == 0 && status_bad(status))) {
                 atomicExch(status, SGB_ERR_TIMEOUT);
                 return false;
             }
+            fetch();
             continue;
         }
 #pragma unroll
@@ -299,7 +298,6 @@ __device__ __forceinline__ bool trsm_row_vals(T* rp, int w, const T* vc, int32_t
             }
         }
         if (tx >= k && tx < k + navail) {
-            T d;
             if (rd != Staged<T>::kSentinel) {
                 d = Staged<T>::val(rd);
             } else {
@@ -309,11 +307,17 @@ __device__ __forceinline__ bool trsm_row_vals(T* rp, int w, const T* vc, int32_t
                 if (!stage_take<T, 1>(dp, want, dv, spin, status)) atomicExch(status, SGB_ERR_TIMEOUT);
                 d = dv[0];
             }
-            const T x = y * rsq<T>(d);
-            stage_put(stage_row + tx, x);
-            rp[tx] = x;
         }
         k += navail;
+        if (k < w) fetch();  // in flight during the square roots
+        if ((k & 7) == 0 || k == w) {
+            const int k0 = (k - 1) & ~7;
+            if (tx >= k0 && tx < k) {
+                const T x = y * rsq<T>(d);
+                stage_put(stage_row + tx, x);
+                rp[tx] = x;
+            }
+        }
     }
     return true;
 }
@@ -364,7 +368,6 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
     // A dependent launch comes in as this grid's CTAs leave: let in at the
     // start, its CTAs settled on a few SMs while this grid held one CTA of every
     // SM, and the product after an FP32 panel at b = 130 took 8 us longer.
-    unsigned* F = a.bar + 0;
     unsigned* I = a.bar + 1;
     unsigned* barB = a.bar + 4;
     unsigned* CC = a.bar + 8;
@@ -386,17 +389,16 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
         for (int64_t p = 0; p < nt; ++p) {
             const int64_t c0 = p * kTile;
             const int w = tile_w(p);
-            if (p >= 3 && !wait_count(I, (unsigned)(p - 2), a.status, &S.flag, a.spin)) return;  // buffer p % 3 free
-                const int buf = (int)(p % 3);
+            const int buf = (int)(p % 3);
             // tile p >= 1 arrives by value from the helpers (their update
-            // with column block p-1); tile-row staging p-1 is then free
+            // with column block p-1); tile-row staging p-1 is then free.  A
+            // wait that gives up sets the status word; the waits of the tiles
+            // left then end at once.
             factor_tile_m<T>(S, a.diag + c0 * a.ldd + c0, a.ldd, w, a.info, a.row0 + c0, Mg + buf * kTile * kTile,
-                             dg + buf * kTile, rg + buf * kTile, CC, (unsigned)(p * kTile),
-                             p >= 1 ? stT + (p & 1) * kTile * kTile : nullptr,
+                             dg + buf * kTile, rg + buf * kTile, CC, (unsigned)(p * kTile), I,
+                             p >= 3 ? (unsigned)(p - 2) : 0u, p >= 1 ? stT + (p & 1) * kTile * kTile : nullptr,
                              p >= 1 ? stL + ((p - 1) & 1) * kTile * kTile : nullptr, a.status, stV + (p % 3) * kVc,
                              p >= 1 ? stV + ((p - 1) % 3) * kVc : nullptr, a.spin);
-            if (!cta_ok(a.status, &S.flag)) return;
-            signal(F);
         }
         return;
     }
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
         for (int64_t p = 0; p < nt; ++p) {
             const int64_t c0 = p * kTile;
             const int w = tile_w(p);
-                if (!wait_count(F, (unsigned)(p + 1), a.status, &S.flag, a.spin)) return;
+            if (!wait_count(CC, (unsigned)(c0 + w), a.status, &S.flag, a.spin)) return;
             const int buf = (int)(p % 3);
             {
                 const T* mt = Mg + buf * kTile * kTile;
@@ -460,16 +462,22 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
             bool took = true;
             if (ty < kHelpRows) {
                 const int r = h * kHelpRows + ty;
-                if (r < w2)
-                    trsm_row_vals<T>(a.diag + (c1 + r) * a.ldd + c0, w, stV + (p % 3) * kVc, a.status, sL + r * kTile,
-                                     a.spin);
+                if (r < w2) {
+                    T* rp = a.diag + (c1 + r) * a.ldd + c0;
+                    trsm_row_vals<T>(rp, p == 0 ? ldcg(rp + tx) : S.x[ty][tx], w, stV + (p % 3) * kVc, a.status,
+                                     sL + r * kTile, a.spin);
+                }
             } else {
                 const int gt = tid - 128, rr1 = h * kHelpRows + ty - 4, cc1 = tx;
-                // this thread's element of tile (p+1, p+1) (last written by this CTA)
+                // this thread's element of tile (p+1, p+1) through step p-1, whose
+                // share is still due (rows of tile-row p+1 in column block p-1
+                // in S.s); the tile itself was last written by the workers
                 const bool own1 = rr1 < w2 && cc1 <= rr1;
-                const T cold = own1 ? ldcg(a.diag + (c1 + rr1) * a.ldd + c1 + cc1) : T(0);
+                T cold = own1 ? ldcg(a.diag + (c1 + rr1) * a.ldd + c1 + cc1) : T(0);
                 T a0 = T(0), a1 = T(0);
                 for (int k0 = 0; k0 < kTile; k0 += 8) {  // (a CTA without rows there must not wait: the buffer is reset)
+                    // (by now the rows wait for columns and leave the FP64 units room)
+                    if (p > 0 && k0 == kTile / 2) cold -= dot32<T>(&S.s[rr1][0], &S.s[cc1][0], kTile);
                     const T* sp[2];
                     bool want[2];
                     T v[2];
@@ -497,20 +505,29 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
             }
             // after the bulk TRSM: column block p applied to their rows of tile-row p+2
             if (!group_barrier(barB, G - 2, epB, a.status, &S.flag, a.spin)) return;
+            // The helpers' way from the barrier to the end of the next rows is
+            // as long as a tile's pivots; with both tiles and a fence here it
+            // was 3 us longer than it is and the factorizer waited for it
+            // (n = b = 512 mixed 141.4 -> 139.8 ms, FP32 b = 130 workflow 5.57
+            // -> 5.41 ms).
+            // (tile (p+2, p+1) now, all warps, half the products each; it stays in S.x,
+            // where the next step's rows start from.  Tile (p+2, p+2) waits for
+            // warps 4-7 of the next step, off the chain.)
             if (has_next2) {
                 load_block<T>(S.s, a.diag + c2 * a.ldd + c0, a.ldd, w3, w);  // L_{p+2,p}
+                const int half = ty >> 2, row = ty & 3, rr = h * kHelpRows + row;
+                const T cold = half == 0 && rr < w3 && tx < w2 ? ldcg(a.diag + (c2 + rr) * a.ldd + c1 + tx) : T(0);
                 __syncthreads();
-                const int half = ty >> 2, rr = h * kHelpRows + (ty & 3), c = tx;
-                if (rr < w3) {
-                    if (half == 0 && c < w2) {  // tile (p+2, p+1)
-                        T* cp = a.diag + (c2 + rr) * a.ldd + c1 + c;
-                        *cp = ldcg(cp) - dot32<T>(&S.s[rr][0], &S.tmp[c][0], w);
-                    } else if (half == 1 && c <= rr) {  // tile (p+2, p+2), lower
-                        T* cp = a.diag + (c2 + rr) * a.ldd + c2 + c;
-                        *cp = ldcg(cp) - dot32<T>(&S.s[rr][0], &S.s[c][0], w);
-                    }
+                T p0 = T(0), p1 = T(0);  // the sums of dot32, two of its four each
+#pragma unroll
+                for (int k = 2 * half; k < kTile; k += 4) {
+                    p0 = fma(S.s[rr][k], S.tmp[tx][k], p0);
+                    p1 = fma(S.s[rr][k + 1], S.tmp[tx][k + 1], p1);
                 }
-                __threadfence();
+                const T part = p0 + p1;
+                if (half == 1) S.u[row][tx] = part;
+                __syncthreads();
+                if (half == 0) S.x[row][tx] = cold - (part + S.u[row][tx]);
                 __syncthreads();
             }
             continue;

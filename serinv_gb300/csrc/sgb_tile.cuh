@@ -496,10 +496,15 @@ __device__ __forceinline__ void tile_columns(Smem<float>& S, int w) {
     if (lane == 0 && fail <= kTile) atomicMin(&S.fail, fail);
 }
 
+__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // The pipeline part of factor_tile alone, for the persistent column-block
 // kernel: after it, S.x holds the strict lower part of M (zero elsewhere)
-// and S.yv the pivots d (1 beyond nb), so L = M diag(d)^{1/2}; no inverse,
-// no output.  FP32 tiles: warps 0-3 take eight columns each (tile_columns).
+// and S.yv the pivots d, so L = M diag(d)^{1/2}; no inverse, no output.  FP32 tiles: warps 0-3 take eight columns each (tile_columns).
 // FP64: the sequential chain is split between two warps on different SM
 // quarters so that each carries as few FP64 instructions as possible:
 //
@@ -514,34 +519,34 @@ __device__ __forceinline__ void tile_columns(Smem<float>& S, int w) {
 //   pivot warp (q_{j+2}, e_{j+2}) -- four FP64 instructions per column;
 // * warps 2, 3, 6, 7 (quarters 2 and 3) apply column k to the strict lower
 //   part of columns k+2.. (the companion keeps the diagonal), then UPD;
-// * with `mt` set, warp 4 publishes the factor outside the pipeline: the
-//   companion counts its finished columns in S.pub (release at CTA scope);
-//   the publisher takes every column finished since its last pass --
+// * warp 4 publishes the factor outside the pipeline, once *free_count has
+//   reached free_target (its buffers are read no more): S.pub counts the
+//   finished columns (release at CTA scope); the publisher takes every column finished since its last pass --
 //   column k of M to mt[k][0..31] (transposed, so a column is one coalesced
 //   row), d_k to dv[k] and d_k^{-1/2} to rv[k] -- makes them visible at GPU
 //   scope and sets *colcount = col_base + (columns published), so other
-//   CTAs consume the columns as they appear.  Its GPU-scope fences never
-//   hold up the pivot pipeline; the chunks grow when a fence is slow.
+//   CTAs consume the columns as they appear.  Its GPU-scope fences do not
+//   hold up the pivot pipeline; the chunks grow when a fence is slow, and the
+//   last one's is waited for while the other warps already take the next tile.
 //
 // With `staged` the tile's lower part comes from that 32 x 32 staging
 // buffer (ld 32) instead of `tile`, each element taken as its producer
 // stores it and reset to the sentinel; `clear` (32 x 32) is reset to the
 // sentinel; a poll that gives up (after `spin` rounds) sets *status =
-// SGB_ERR_TIMEOUT.  With
-// `vcols` warp 5 also hands the factor on by value, without fences: d_k to
-// vcols[1024 + k] and column k of M to vcols[32 k .. 32 k + 31] as the
-// companion finishes them; `vclear` (32 x 32 + 32) is reset first.
+// SGB_ERR_TIMEOUT.  Without, it is the launch's first tile.  Warp 5 also hands
+// the factor on by value, without fences: d_k to vcols[1024 + k] and column k
+// of M to vcols[32 k .. 32 k + 31] as they are finished; `vclear` (32 x 32 + 32)
+// is reset first.
 //
 // Pivot <-> companion hand-offs use named barriers PQ (ids 5, 6) and QP
 // (7, 8), READY/UPD ids 1-4 (companion + workers); every pair alternates
 // between two ids so that no side can run two generations ahead (the
 // arrival sequence was checked on a CPU model for nb = 1..32).
 template <typename T>
-__device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int32_t* info, int64_t row0,
-                              T* mt = nullptr, T* dv = nullptr, T* rv = nullptr, unsigned* colcount = nullptr,
-                              unsigned col_base = 0, T* staged = nullptr, T* clear = nullptr,
-                              int32_t* status = nullptr, T* vcols = nullptr, T* vclear = nullptr,
-                              long long spin = 1ll << 22) {
+__device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int32_t* info, int64_t row0, T* mt,
+                              T* dv, T* rv, unsigned* colcount, unsigned col_base, const unsigned* free_count,
+                              unsigned free_target, T* staged, T* clear, int32_t* status, T* vcols, T* vclear,
+                              long long spin) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int kCons = 32 * 5;  // companion + four workers
     constexpr int kPair = 64;
@@ -549,6 +554,19 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
     T* qv = &S.tmp[1][0];  // a'_{j,j-1}^2
     T* ev = &S.tmp[2][0];  // diagonal of column j through column j-2
     constexpr int U = kTile * kTile / kTileThreads;
+    constexpr bool kRegs = sizeof(T) == 4;
+    if (staged == nullptr) {  // the first tile of the launch: what the later ones keep
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = tid + u * kTileThreads, r = e / kTile, c = e % kTile;
+            S.x[r][c] = T(0);
+            if (c < r) S.tri[r * (r - 1) / 2 + c] = (unsigned short)((r << 8) | c);  // strict lower, row-major
+        }
+    }
+    if (tid == 0) {
+        S.fail = kRegs ? kTile + 1 : 0;
+        S.pub = 0;
+    }
     bool timed_out = false;
     T sv[U];
     if (staged != nullptr) {  // lower part of the tile as its producers store it
@@ -561,9 +579,6 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
             want[u] = r < nb && c <= r;
         }
         timed_out = !stage_take<T, U>(sp, want, sv, spin, status);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (want[u]) stage_clear(staged + tid + u * kTileThreads);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -572,17 +587,11 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
         if (r < nb && c <= r) v = staged != nullptr ? sv[u] : __ldcg(tile + (int64_t)r * ld + c);
         else if (r >= nb && r == c) v = T(1);
         S.s[r][c] = v;
-        S.x[r][c] = T(0);
-        if (c < r) S.tri[r * (r - 1) / 2 + c] = (unsigned short)((r << 8) | c);  // strict lower, row-major
+        if (staged != nullptr && r < nb && c <= r) stage_clear(staged + e);
     }
-    if (tid < kTile) S.yv[tid] = T(1);
-    constexpr bool kRegs = sizeof(T) == 4;
-    if (tid == 0) {
-        S.fail = kRegs ? kTile + 1 : 0;
-        S.pub = 0;
-    }
-    if (timed_out && status != nullptr) atomicExch(status, SGB_ERR_TIMEOUT);
+    if (timed_out) atomicExch(status, SGB_ERR_TIMEOUT);
     __syncthreads();
+    bool last_unseen = false;  // warp 4: the tile's last columns are stored but not made visible yet
     if (kRegs && warp < 4) {
         // (columns from nb on are those of the identity)
         if constexpr (kRegs)
@@ -622,11 +631,10 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
             const T mcol = col * inv;
             if (lane >= j) S.s[lane][j] = col;
             if (lane > j) S.x[lane][j] = mcol;
-            if (mt != nullptr) {  // column j (and d_j, seen through PQ(j)) to the publisher
-                __syncwarp();
-                if (lane == 0) asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(&S.pub)), "r"(j + 1)
-                                            : "memory");
-            }
+            // column j (and d_j, seen through PQ(j)) to the publisher
+            __syncwarp();
+            if (lane == 0) asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(&S.pub)), "r"(j + 1)
+                                        : "memory");
             nbar_arrive(1 + (j & 1), kCons);  // READY(j)
             if (j >= 1) nbar_sync(3 + ((j - 1) & 1), kCons);  // UPD(j-1)
             if (j + 1 < nb) {
@@ -644,28 +652,41 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
             }
         }
     } else if (warp == 4) {
-        if (mt != nullptr) {
-            int done = 0;
-            long long spins = 0;
-            while (done < nb) {
-                int avail = 0;
-                for (;;) {  // bounded: the companion finishes every column in any case
-                    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(avail) : "r"(smem_u32(&S.pub)) : "memory");
-                    if (avail > done || ++spins > (1ll << 26)) break;
+        // the L writer has read these buffers (three tiles ago)
+        if (lane == 0 && free_target > 0) {
+            long long polls = 0;
+            while (ld_acquire_gpu(free_count) < free_target) {
+                if (++polls > spin || ((polls & 63) == 0 && *(const volatile int32_t*)status != 0)) {
+                    atomicExch(status, SGB_ERR_TIMEOUT);
+                    break;
                 }
-                if (avail <= done) break;  // the waits of the consumers time out and report it
-                avail = avail < nb ? avail : nb;
-                for (int k = done; k < avail; ++k) mt[k * kTile + lane] = S.x[lane][k];
-                if (lane >= done && lane < avail) {
-                    const T d = S.yv[lane];
-                    dv[lane] = d;
-                    rv[lane] = rsq<T>(d);
-                }
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) atomicExch(colcount, col_base + (unsigned)avail);
-                done = avail;
             }
+        }
+        __syncwarp();
+        int done = 0;
+        long long spins = 0;
+        while (done < nb) {
+            int avail = 0;
+            for (;;) {  // bounded: the companion finishes every column in any case
+                asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(avail) : "r"(smem_u32(&S.pub)) : "memory");
+                if (avail > done || ++spins > (1ll << 26)) break;
+            }
+            if (avail <= done) break;  // the waits of the consumers time out and report it
+            avail = avail < nb ? avail : nb;
+            for (int k = done; k < avail; ++k) mt[k * kTile + lane] = S.x[lane][k];
+            if (lane >= done && lane < avail) {
+                const T d = S.yv[lane];
+                dv[lane] = d;
+                rv[lane] = rsq<T>(d);
+            }
+            done = avail;
+            if (done == nb) {  // this one's fence does not hold up the CTA
+                last_unseen = true;
+                break;
+            }
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) atomicExch(colcount, col_base + (unsigned)avail);
         }
     } else if (warp == 5) {
         // every consumer of `clear` and `vclear` is done with them (they all
@@ -674,23 +695,21 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
             for (int e = lane; e < kTile * kTile; e += 32) stage_clear(clear + e);
         if (vclear != nullptr)
             for (int e = lane; e < kTile * kTile + kTile; e += 32) stage_clear(vclear + e);
-        if (vcols != nullptr) {
-            // the columns by value as the companion finishes them: d_k to
-            // vcols[1024 + k], then column k of M to vcols[k * 32 + 0..31]
-            int done = 0;
-            long long spins = 0;
-            while (done < nb) {
-                int avail = 0;
-                for (;;) {
-                    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(avail) : "r"(smem_u32(&S.pub)) : "memory");
-                    if (avail > done || ++spins > (1ll << 26)) break;
-                }
-                if (avail <= done) break;
-                avail = avail < nb ? avail : nb;
-                if (lane >= done && lane < avail) stage_put(vcols + kTile * kTile + lane, S.yv[lane]);
-                for (int k = done; k < avail; ++k) stage_put(vcols + k * kTile + lane, S.x[lane][k]);
-                done = avail;
+        // the columns by value as the companion finishes them: d_k to
+        // vcols[1024 + k], then column k of M to vcols[k * 32 + 0..31]
+        int done = 0;
+        long long spins = 0;
+        while (done < nb) {
+            int avail = 0;
+            for (;;) {
+                asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(avail) : "r"(smem_u32(&S.pub)) : "memory");
+                if (avail > done || ++spins > (1ll << 26)) break;
             }
+            if (avail <= done) break;
+            avail = avail < nb ? avail : nb;
+            if (lane >= done && lane < avail) stage_put(vcols + kTile * kTile + lane, S.yv[lane]);
+            for (int k = done; k < avail; ++k) stage_put(vcols + k * kTile + lane, S.x[lane][k]);
+            done = avail;
         }
     } else if (!kRegs) {
         const int wid = (warp < 4 ? warp - 2 : warp - 4) * 32 + lane;  // 0..127
@@ -707,6 +726,11 @@ __device__ void factor_tile_m(Smem<T>& S, const T* tile, int64_t ld, int nb, int
         }
     }
     __syncthreads();
+    if (last_unseen) {
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicExch(colcount, col_base + (unsigned)nb);
+    }
     if (tid == 0 && S.fail != (kRegs ? kTile + 1 : 0) && info != nullptr) atomicCAS(info, 0, (int32_t)(row0 + S.fail));
 }
 
