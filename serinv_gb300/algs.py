@@ -364,16 +364,19 @@ def pobtaf(A_diagonal_blocks, A_lower_diagonal_blocks, A_lower_arrow_blocks, A_a
         _lib.raise_for(lib.sgb_pobtaf_workspace_size(ctypes.byref(m), precision, ctypes.byref(nbytes)),
                        "pobtaf")
         ws = _workspace(nbytes.value, device)
-        info = torch.zeros(1, dtype=torch.int32, device=device)
+        # the second word of the status slot, set by the call itself: one read
+        # tells both, and no buffer is made and cleared for it
         rc = lib.sgb_pobtaf(ctypes.byref(m), int(factorize_last_block), precision, ws.data_ptr(),
-                            nbytes.value, info.data_ptr(), _stream(device))
+                            nbytes.value, ws.data_ptr() + 4, _stream(device))
         _lib.raise_for(rc, "pobtaf")
         _finish(w)
-        _check_status(ws, precision, "pobtaf", always=check)
         if check:
-            k = int(info.item())
+            code, k = ws[:8].view(torch.int32).tolist()
+            _lib.raise_for(code, "pobtaf")
             if k > 0:
                 raise np.linalg.LinAlgError(f"{k}-th leading minor of the array is not positive definite")
+        else:
+            _check_status(ws, precision, "pobtaf")
 
 
 def pobtasi(L_diagonal_blocks, L_lower_diagonal_blocks, L_lower_arrow_blocks, L_arrow_tip_block, **kwargs):
