@@ -94,6 +94,14 @@ constexpr int64_t kExactMinFactor = 240, kExactMinInverse = 224;
 // holds K <= kTcMaxK.
 bool inverse_form(int64_t b) { return b > 2 * kTile && ceil_div(b, 32) * 32 <= kTcMaxK; }
 
+// Column blocks of such a factorization from this size on are factored in two
+// halves: the update of the second half's columns by the first (44 % of the FP64
+// work at b = 512) is then one product on the tensor cores, which costs 30 us with
+// the second launch.  us a block, whole and halves: b = 400 243 and 247, b = 448
+// 294 and 284, b = 480 310 and 290, b = 512 372 and 324; against 64 bits 7.7e-16
+// and 5.4e-16 at b = 512.
+constexpr int64_t kPanelHalves = 416;
+
 // The slice count of a native FP64 sweep, or 0: the FP64 pipe.
 int exact_slices(const sgb_bta* m, bool inverse) {
     return m->dtype == SGB_F64 && m->b >= (inverse ? kExactMinInverse : kExactMinFactor) &&
@@ -779,6 +787,38 @@ int pobtaf_run(const sgb_bta* m, int factorize_last_block, int S, int Si, void* 
             }
             if (e != cudaErrorNotSupported) return cuda_fail(e);
             mixed_inverse = false;  // too few SMs for the persistent launch
+        }
+        if (persistent && S == kExactSlices && b >= kPanelHalves) {
+            // [D_i; Lo_i; Ar_i] in two halves of its columns, with one product on
+            // the tensor cores between them
+            const int64_t h = ceil_div(b / 2, (int64_t)kTile) * kTile, h2 = b - h;
+            cudaError_t e = factor_panel_persistent<T>(Di, h, b, r1, r2, tinv, bar, cx.status, info, i * b, s, nullptr,
+                                                       pgrid, h2);
+            if (e == cudaSuccess) {
+                T* D21 = Di + h * b;
+                GemmProb<T> pr[3];
+                int np = 0;
+                for (RowSet<T> r : {RowSet<T>{D21, h2, b}, r1, r2}) {
+                    if (r.rows <= 0 || r.p == nullptr) continue;
+                    GemmProb<T> p = prob<T>();  // columns h .. -= columns .. h times D21^T
+                    p.M = (int32_t)r.rows;
+                    p.N = (int32_t)h2;
+                    set_term<T>(p, 0, r.p, r.ld, 0, D21, b, 1, h);
+                    p.alpha = T(-1);
+                    p.beta = T(1);
+                    p.Cin = p.Cout = r.p + h;
+                    p.ldcin = p.ldc = r.ld;
+                    p.lower_only = r.p == D21 ? 1 : 0;
+                    pr[np++] = p;
+                }
+                SGB_TRY(run_gemm<T>(cx, pr, np, s));
+                for (RowSet<T>* r : {&r1, &r2})
+                    if (r->p != nullptr) r->p += h;
+                e = factor_panel_persistent<T>(D21 + h, h2, b, r1, r2, tinv, bar, cx.status, info, i * b + h, s, nullptr,
+                                               pgrid);
+                return e == cudaSuccess ? SGB_OK : cuda_fail(e);
+            }
+            if (e != cudaErrorNotSupported) return cuda_fail(e);
         }
         cudaError_t e = persistent ? factor_panel_persistent<T>(Di, b, b, r1, r2, tinv, bar, cx.status, info, i * b,
                                                                 s, nullptr, pgrid)

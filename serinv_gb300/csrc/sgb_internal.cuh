@@ -129,11 +129,13 @@ using GemmFn = cudaError_t (*)(void* ctx, GemmProb<T>* probs, int np, cudaStream
 // the caller zeroes them once.  Not for use under stream capture
 // (cooperative launch).
 // `grid_cap` > 0 limits the grid (a launch captured beside others in a
-// graph takes only part of the GPU).
+// graph takes only part of the GPU).  `below`: D has that many rows (and
+// columns) more; the rows are solved like the row sets', the columns zeroed
+// beside the factored tiles (m a multiple of kTile then).
 template <typename T>
 cudaError_t factor_panel_persistent(T* diag, int64_t m, int64_t ldd, RowSet<T> r1, RowSet<T> r2, T* tinv,
                                     unsigned* bar, int32_t* status, int32_t* info, int64_t info_row0,
-                                    cudaStream_t s, T* xinv = nullptr, int grid_cap = 0);
+                                    cudaStream_t s, T* xinv = nullptr, int grid_cap = 0, int64_t below = 0);
 
 // Grid of the column-block kernel in sweeps captured by this host thread
 // (0: captured sweeps use the launch-based tile sweep).  Batch plans set it

@@ -68,6 +68,9 @@ template <typename T>
 struct PanelArgs {
     T* diag;
     int64_t m, ldd;
+    int64_t mz;  // columns of D: those right of a diagonal tile are set to zero
+    T* r0;  // rows of D below the m factored columns' own
+    int64_t r0rows;
     T* r1;
     int64_t r1rows, r1ld;
     T* r2;
@@ -165,12 +168,14 @@ __device__ __forceinline__ void signal(unsigned* ctr) {
     }
 }
 
-// Row r of the unified row space [D rows c1..m) ++ r1 rows ++ r2 rows.
+// Row r of the unified row space [D rows c1..m) ++ r0 rows ++ r1 rows ++ r2 rows.
 template <typename T>
 __device__ __forceinline__ T* row_ptr(const PanelArgs<T>& a, int64_t c1, int64_t r) {
     const int64_t nd = a.m - c1;
     if (r < nd) return a.diag + (c1 + r) * a.ldd;
     r -= nd;
+    if (r < a.r0rows) return a.r0 + r * a.ldd;
+    r -= a.r0rows;
     if (r < a.r1rows) return a.r1 + r * a.r1ld;
     return a.r2 + (r - a.r1rows) * a.r2ld;
 }
@@ -418,7 +423,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                 S.tmp[0][tid] = ldcg(rg + buf * kTile + tid);
             }
             __syncthreads();
-            tile_l_from_m<T>(S.x, S.yv, &S.tmp[0][0], a.diag + c0 * a.ldd + c0, a.ldd, w, (int)(m - c0 - w));
+            tile_l_from_m<T>(S.x, S.yv, &S.tmp[0][0], a.diag + c0 * a.ldd + c0, a.ldd, w, (int)(a.mz - c0 - w));
             signal(I);
         }
         return;
@@ -554,7 +559,7 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
         const int nwk = (int)G - kW0, wk = (int)cta - kW0;
         const bool prev = p >= 1;  // the trailing update of step p-1 is due
         const int64_t off0 = w2;
-        const int64_t nbase = (m - c1) + a.r1rows + a.r2rows - off0;
+        const int64_t nbase = (m - c1) + a.r0rows + a.r1rows + a.r2rows - off0;
         const int64_t nrows = nbase + (a.xinv ? c1 : 0);
         if (tid == 0) S.rowq[(p + 1) & 1] = 0;  // the next step's row counter (used after barrier B)
         // Rows go to the CTAs four at a time.  Warps 0-3 start with q = ty and take every further q from a shared
@@ -568,10 +573,11 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
         // with cj >= 1.
         const int64_t c0q = c0 - kTile, c1q = c0;
         const int ntd = (int)((m - c1q + kTile - 1) / kTile);  // tile-rows from tile-row p
+        const int n0 = (int)((a.r0rows + kTile - 1) / kTile);
         const int n1 = (int)((a.r1rows + kTile - 1) / kTile), n2 = (int)((a.r2rows + kTile - 1) / kTile);
         const int nx = a.xinv ? (int)p : 0;
         const int tiles_d = ntd >= 2 ? ntd * (ntd - 1) / 2 - 1 : 0;
-        const int total = prev && ntd >= 2 ? tiles_d + (n1 + n2 + nx) * (ntd - 1) : 0;
+        const int total = prev && ntd >= 2 ? tiles_d + (n0 + n1 + n2 + nx) * (ntd - 1) : 0;
         // An FP64 tile keeps a worker's FP64 units (64 cycles a warp
         // instruction and SM quarter) busy for 8 us, so where halves leave a
         // shorter last round the workers take half tiles: n=128 b=512 with 390
@@ -667,20 +673,26 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                     const int u = t - tiles_d;
                     const int set = u / (ntd - 1);
                     R.cj = 1 + (u - set * (ntd - 1));
-                    if (set < n1) {
+                    if (set < n0) {
                         ti = set;
+                        R.C = a.r0 + ti * kTile * a.ldd + c1q;
+                        R.A = a.r0 + ti * kTile * a.ldd + c0q;
+                        R.ldc = a.ldd;
+                        R.rows = a.r0rows - ti * kTile;
+                    } else if (set < n0 + n1) {
+                        ti = set - n0;
                         R.C = a.r1 + ti * kTile * a.r1ld + c1q;
                         R.A = a.r1 + ti * kTile * a.r1ld + c0q;
                         R.ldc = a.r1ld;
                         R.rows = a.r1rows - ti * kTile;
-                    } else if (set < n1 + n2) {
-                        ti = set - n1;
+                    } else if (set < n0 + n1 + n2) {
+                        ti = set - n0 - n1;
                         R.C = a.r2 + ti * kTile * a.r2ld + c1q;
                         R.A = a.r2 + ti * kTile * a.r2ld + c0q;
                         R.ldc = a.r2ld;
                         R.rows = a.r2rows - ti * kTile;
                     } else {
-                        ti = set - n1 - n2;
+                        ti = set - n0 - n1 - n2;
                         R.C = a.xinv + ti * kTile * a.xld + c1q;
                         R.A = a.xinv + ti * kTile * a.xld + c0q;
                         R.ldc = a.xld;
@@ -805,7 +817,7 @@ int g_panel_grid[64] = {};
 template <typename T>
 cudaError_t factor_panel_persistent(T* diag, int64_t m, int64_t ldd, RowSet<T> r1, RowSet<T> r2, T* tinv,
                                     unsigned* bar, int32_t* status, int32_t* info, int64_t info_row0,
-                                    cudaStream_t s, T* xinv, int grid_cap) {
+                                    cudaStream_t s, T* xinv, int grid_cap, int64_t below) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -825,6 +837,9 @@ cudaError_t factor_panel_persistent(T* diag, int64_t m, int64_t ldd, RowSet<T> r
     a.diag = diag;
     a.m = m;
     a.ldd = ldd;
+    a.mz = m + below;
+    a.r0 = diag + m * ldd;
+    a.r0rows = below;
     a.r1 = r1.p;
     a.r1rows = r1.p ? r1.rows : 0;
     a.r1ld = r1.ld;
@@ -852,16 +867,16 @@ cudaError_t factor_panel_persistent(T* diag, int64_t m, int64_t ldd, RowSet<T> r
     // (+ the triangular inverse)
     const double md = (double)m;
     prof_after(SGB_KCLASS_PANEL, s,
-               md * md * md / 3.0 * (xinv ? 2.0 : 1.0) + (double)(a.r1rows + a.r2rows) * md * md);
+               md * md * md / 3.0 * (xinv ? 2.0 : 1.0) + (double)(below + a.r1rows + a.r2rows) * md * md);
     return e;
 }
 
 template cudaError_t factor_panel_persistent<double>(double*, int64_t, int64_t, RowSet<double>, RowSet<double>,
                                                      double*, unsigned*, int32_t*, int32_t*, int64_t, cudaStream_t,
-                                                     double*, int);
+                                                     double*, int, int64_t);
 template cudaError_t factor_panel_persistent<float>(float*, int64_t, int64_t, RowSet<float>, RowSet<float>,
                                                     float*, unsigned*, int32_t*, int32_t*, int64_t, cudaStream_t,
-                                                    float*, int);
+                                                    float*, int, int64_t);
 
 namespace {
 thread_local int t_capture_panel_grid = 0;

@@ -49,3 +49,30 @@ def test_first_bad_pivot(bad, dtype):
     d = [torch.from_numpy(x).cuda() for x in (D, np.zeros((2, b, b), dtype))]
     with pytest.raises(np.linalg.LinAlgError, match=f"^{b + min(bad) + 1}-th"):
         sg.pobtf(*d)
+
+
+# FP64 column blocks in two halves (from b = 416 on; 576: the longest product of the exact form)
+@pytest.mark.parametrize("b,a", [(415, 3), (416, 0), (417, 64), (449, 33), (500, 1), (576, 130)])
+@pytest.mark.parametrize("last", [True, False])
+def test_halves(b, a, last):
+    m = generate(2, b, a, 1, seed=b)
+    d = [torch.from_numpy(x.copy()).cuda() for x in m.arrays()]
+    ref = [x.copy() for x in m.arrays()]
+    sg.pobtaf(*d, factorize_last_block=last)
+    oracle.pobtaf(*ref, factorize_last_block=last)
+    got = [x.cpu().numpy() for x in d]
+    if not last:  # of what is left unfactored the lower triangles are defined
+        got[0][-1], ref[0][-1] = np.tril(got[0][-1]), np.tril(ref[0][-1])
+        got[3], ref[3] = np.tril(got[3]), np.tril(ref[3])
+    for x, y in zip(got, ref):
+        assert np.linalg.norm(x - y) <= 1e-12 * max(np.linalg.norm(y), 1e-300)
+
+
+@pytest.mark.parametrize("bad", [100, 223, 224, 300, 430])
+def test_halves_first_bad_pivot(bad):
+    D = np.repeat(4 * np.eye(431)[None], 2, 0)
+    D[:, 1:, :-1] += np.eye(430)
+    D[0, bad, bad] = -1
+    d = [torch.from_numpy(x).cuda() for x in (D, np.zeros((1, 431, 431)))]
+    with pytest.raises(np.linalg.LinAlgError, match=f"^{bad + 1}-th"):
+        sg.pobtf(*d)
