@@ -33,7 +33,7 @@ from .algs import _bta_struct
 
 _OPS = {"pobtaf": 1, "pobtasi": 2, "pobtas": 4}
 CANDIDATES = (8, 16, 32, 64, 128)
-PANEL_CANDIDATES = (18, 24, 32)
+PANEL_CANDIDATES = (18, 32, 64)  # beside the default, 48
 CACHE = os.environ.get("SGB_AUTOTUNE_CACHE",
                        os.path.join(os.path.expanduser("~"), ".cache", "serinv_gb300", "batch_autotune.json"))
 
@@ -150,7 +150,7 @@ def autotune(mats, rhs=None, ops=("pobtaf", "pobtasi", "pobtas"), precisions=Non
              panel_candidates=PANEL_CANDIDATES, reps: int = 2):
     """Pick (worker-stream count, column-block CTA count, tensor-core K
     split) by timing warm replays on scratch copies of the batch: the stream
-    count first (CTA count 24, no K split), then the CTA count at that
+    count first (the default CTA count, no K split), then the CTA count at that
     stream count, then the K split.  Cached by signature."""
     if precisions is None:
         precisions = ["fp64"] * len(mats)
@@ -176,7 +176,7 @@ def autotune(mats, rhs=None, ops=("pobtaf", "pobtasi", "pobtas"), precisions=Non
             best_ns, best_t = ns, t
     best_panel = 0
     for pc in panel_candidates:
-        if pc == 24:  # the stream search ran at 24
+        if pc == 24:  # never the best: between 18 and the default, at which the stream search ran
             continue
         t = _time_plan(mats, rhs, scratch, srhs, ops, precisions, best_ns, pc, reps)
         if t < best_t:

@@ -16,8 +16,13 @@
 
 #include "sgb_internal.cuh"
 
-// CTAs of a captured column-block launch unless the plan asks otherwise.
-constexpr int kPlanPanelGrid = 24;
+// CTAs of a captured column-block launch unless the plan asks otherwise: three
+// launches side by side on 152 SMs.  Ten CTAs of a launch have other roles, so 24
+// left the trailing update of a block to 14.  ms a replay on 12 streams with 24,
+// 40, 48 and 64 CTAs: 12 matrices up to n=96 b=256, half of them FP32, mixed 34.9,
+// 29.7, 29.9, 30.5 and FP64 51.1, 38.8, 36.9, 37.4; 24 up to n=48 mixed 19.6, 18.6,
+// 19.2, 21.3; 4 up to n=40 mixed 14.1, 11.4, 11.2, 10.7.
+constexpr int kPlanPanelGrid = 48;
 
 struct sgb_batch_plan {
     int count = 0;

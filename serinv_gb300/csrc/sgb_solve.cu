@@ -6,7 +6,8 @@
 // FMAs) is small next to what a launch, or a barrier over the whole GPU,
 // costs.  Launched product by product (two or three launches per block, and
 // the full inverse of every diagonal block first) the sweep ran at 86 us per
-// block for b = 512 and one right-hand side and 420 us with sixteen.
+// block for b = 512 and one right-hand side and 420 us with sixteen; as it is 22
+// and 54 us.
 //
 // Here a cluster of G CTAs walks the whole chain and exchanges values through
 // distributed shared memory: asynchronous stores that count their bytes on the
@@ -39,7 +40,7 @@
 // have read y_q.
 //
 // A warp issues one FP64 instruction per 64 cycles, one lane or all, and the
-// SM one per 19: four warps on two rows each (16 lanes per row) give a chain
+// SM one per 16 to 19: four warps on two rows each (16 lanes per row) give a chain
 // step the fewest cycles (12 instructions a warp at k = 128, of which four
 // reduce).  In the bulk update one warp forms RW outputs at once and the
 // reduction halves the outputs a lane carries at every shuffle step (V - 1 +
