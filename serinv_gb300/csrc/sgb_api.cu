@@ -83,11 +83,13 @@ int parse_inv_slices(int precision, int S) {
 // rows and columns scaled by up to 10^+-6 neither changes (the products over
 // rows of an inverse are balanced by its diagonal).  The factorization of the
 // column blocks stays on the FP64 pipe.
-// Below the lines the slicing and the longer epilogue cost more than the FP64
-// pipe's 16 x 16 tiles: selected inverse n=64 (us) b=208 4961 against 4617, b=224
-// 4574 / 5458, b=256 a=32 5561 / 8055, b=512 (n=32) 5618 / 26456; factorization
-// b=224 8787 / 8552, b=240 9441 / 10090, b=512 (n=32) 13522 / 16960.
-constexpr int64_t kExactMinFactor = 240, kExactMinInverse = 224;
+// Below the line the slicing and the longer epilogue cost more than the FP64
+// pipe's 16 x 16 tiles.  us, exact slices and FP64 pipe: selected inverse n=64
+// b=160 a=48 3299 / 3464 but a=0 3036 / 2554, b=176 a=16 3383 / 4103, b=208 3702 /
+// 4599, b=256 a=32 4125 / 8055, b=512 (n=32) 4600 / 26456; factorization n=64
+// b=160 a=0 5943 / 5632, b=176 a=16 6505 / 6703, b=192 a=64 6865 / 7160, b=240 8277
+// / 9164, b=512 (n=32) 10378 / 16960.
+constexpr int64_t kExactMin = 176;
 
 // Whether a mixed factorization may take rows * L_ii^{-T} as a product: in place,
 // which only the tensor-core form does (it slices its operands first), and that
@@ -103,8 +105,8 @@ bool inverse_form(int64_t b) { return b > 2 * kTile && ceil_div(b, 32) * 32 <= k
 constexpr int64_t kPanelHalves = 416;
 
 // The slice count of a native FP64 sweep, or 0: the FP64 pipe.
-int exact_slices(const sgb_bta* m, bool inverse) {
-    return m->dtype == SGB_F64 && m->b >= (inverse ? kExactMinInverse : kExactMinFactor) &&
+int exact_slices(const sgb_bta* m) {
+    return m->dtype == SGB_F64 && m->b >= kExactMin &&
                    ceil_div(m->b, 32) * 32 <= kTcMaxK
                ? kExactSlices
                : 0;
@@ -355,11 +357,11 @@ size_t tasi_bytes(const sgb_bta* m, int S, int Si, int64_t cap = kSiChunk) {
     return m->dtype == SGB_F64 ? PobtasiWs<double>(m, S, Si, cap).total : PobtasiWs<float>(m, S, Si, cap).total;
 }
 int taf_slices(const sgb_bta* m, int S, size_t have) {
-    const int X = S ? 0 : exact_slices(m, false);
+    const int X = S ? 0 : exact_slices(m);
     return X && have >= taf_bytes(m, X, 0) ? X : S;
 }
 int tasi_slices(const sgb_bta* m, int S, size_t have) {
-    const int X = S ? 0 : exact_slices(m, true);
+    const int X = S ? 0 : exact_slices(m);
     return X && have >= tasi_bytes(m, X, 0) ? X : S;
 }
 
@@ -1749,7 +1751,7 @@ int stream_sizes(const sgb_bta* host, int precision, int64_t ring, bool inverse,
     const int Si = parse_inv_slices(precision, S);
     *R = inverse ? ring_slots(ring, kRingPobtasi, true) : ring_slots(ring, kRingPobtaf, false);
     if (*R < 2 || *R > ((int64_t)1 << 20)) return SGB_ERR_SHAPE;
-    for (int X : {S ? S : exact_slices(host, inverse), S}) {
+    for (int X : {S ? S : exact_slices(host), S}) {
         *slices = X;
         *sweep = inverse ? tasi_bytes(host, X, Si, *R / 2) : taf_bytes(host, X, Si);
         *total = StreamWs(host, *sweep, *R).total;
@@ -1792,7 +1794,7 @@ int sgb_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes) {
     if (S < 0) return -S;
     if (!bytes) return SGB_ERR_ARG;
     const int Si = parse_inv_slices(precision, S);
-    *bytes = m->dtype == SGB_F64 ? PobtafWs<double>(m, S ? S : exact_slices(m, false), Si).total
+    *bytes = m->dtype == SGB_F64 ? PobtafWs<double>(m, S ? S : exact_slices(m), Si).total
                                  : PobtafWs<float>(m, S, Si).total;
     return SGB_OK;
 }
@@ -1805,7 +1807,7 @@ int sgb_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes) {
     if (S < 0) return -S;
     if (!bytes) return SGB_ERR_ARG;
     const int Si = parse_inv_slices(precision, S);
-    *bytes = m->dtype == SGB_F64 ? PobtasiWs<double>(m, S ? S : exact_slices(m, true), Si).total
+    *bytes = m->dtype == SGB_F64 ? PobtasiWs<double>(m, S ? S : exact_slices(m), Si).total
                                  : PobtasiWs<float>(m, S, Si).total;
     return SGB_OK;
 }

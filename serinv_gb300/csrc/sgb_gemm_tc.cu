@@ -1163,7 +1163,13 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         if (k > minkb) k = minkb;
         ks = k < 1 ? 1 : (int)k;
     }
-    const int bn = (ks > 1 || tiles64 >= 148) ? 64 : 32;
+    // 128 x 32 tiles also beside the deepest split while twice the CTAs still fit
+    // the SMs: a CTA's MMAs, folding and writing are half as long.  ms at n=64,
+    // factorization / selected inverse: b=256 FP64 8.76 / 4.78 -> 8.40 / 4.13, mixed
+    // 9.39 / 3.42 -> 8.95 / 2.96, b=128 mixed 5.90 / 2.71 -> 5.39 / 2.16; beyond that
+    // a second wave costs more (b=512 FP64 20.5 / 9.1 -> 21.6 / 9.8).
+    const bool narrow = ks == kTcMaxSplit && 2 * tiles64 * ks <= kTcSmCount;
+    const int bn = !narrow && (ks > 1 || tiles64 >= 148) ? 64 : 32;
     TL.ks = ks;
     for (int i = 0; i < np; ++i) {
         const GemmProb<double>& p = probs[i];

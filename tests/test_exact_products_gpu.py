@@ -12,8 +12,8 @@ from serinv_gb300.synthetic import generate
 
 pytestmark = pytest.mark.gpu
 
-# 224 / 240: where the selected inverse / the factorization change over; 576: the longest contraction
-SHAPES = [(3, 223, 5), (3, 224, 0), (3, 240, 33), (4, 257, 64), (2, 300, 1), (3, 544, 32), (2, 576, 0), (2, 577, 3),
+# 176: where the forms change over; 576: the longest contraction
+SHAPES = [(5, 175, 8), (5, 176, 8), (4, 190, 0), (3, 223, 5), (3, 224, 0), (3, 240, 33), (4, 257, 64), (2, 300, 1), (3, 544, 32), (2, 576, 0), (2, 577, 3),
           (1, 320, 40)]
 
 
