@@ -438,9 +438,10 @@ __device__ void factor_tile(Smem<T>& S, T* tile, int64_t ld, int nb, int zero_ri
 // in registers.  An FP32 column has some 20 instructions of arithmetic, and with
 // a warp for the pivots, one for the next column and four for the rest, the two
 // barrier hops of every column took 403 cycles; here a hop lies between two
-// warps' columns only (287 cycles a column with the tile's load and end).  u = a'_ij (rows below the pivot) and
-// v = - u / d_j of every finished column stand in S.u and S.tmp (32 x 32), v as
-// M(:, j) in S.x as well; S.pub counts the columns.
+// warps' columns only (287 cycles a column with the tile's load and end).
+// u = a'_ij (rows below the pivot) and v = - u / d_j of every finished column
+// stand in S.u and S.tmp (32 x 32), v as M(:, j) in S.x as well; S.pub counts the
+// columns.
 __device__ __forceinline__ void tile_columns(Smem<float>& S, int w) {
     constexpr int W = kTile / 4;
     const int lane = threadIdx.x & 31, c0 = w * W;
