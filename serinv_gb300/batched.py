@@ -33,7 +33,7 @@ from .algs import _bta_struct
 
 _OPS = {"pobtaf": 1, "pobtasi": 2, "pobtas": 4}
 CANDIDATES = (8, 16, 32, 64, 128)
-PANEL_CANDIDATES = (18, 32, 64)  # beside the default, 48
+PANEL_CANDIDATES = (18, 26, 34, 64)  # beside the default, 48
 CACHE = os.environ.get("SGB_AUTOTUNE_CACHE",
                        os.path.join(os.path.expanduser("~"), ".cache", "serinv_gb300", "batch_autotune.json"))
 
