@@ -392,18 +392,19 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
             const T* Cn = last_block ? nullptr : coupling(j);
             for (int qi = 0; qi < cur.nsub; ++qi, ++step) {
                 const int q = tr ? cur.nsub - 1 - qi : qi;
-                const bool last_q = qi == cur.nsub - 1;
+                const bool last_q = qi == cur.nsub - 1, end = last_block && last_q;
                 const int K0 = q * cur.s, K = cur.rows(q);
                 const unsigned p = step & 1, ph = (step >> 1) & 1;
                 T* y = (tr && j == a.n) ? ytip + (size_t)K0 * NR : ybuf + p * kBuf;
                 // credits land behind the rows (behind all of the tip's)
                 T* ycr = (tr && j == a.n) ? ytip + (size_t)a.a * NR : y + kSub * NR;
-                if (tid == 0) bar_expect(by + p, xbytes(cur, q));
+                // nobody reads the last y: it is not exchanged (see the end of the kernel)
+                if (tid == 0 && !end && !*fail) bar_expect(by + p, xbytes(cur, q));
                 // y_q = Linv_qq x_q, own rows
                 if (step > 0) bar_wait(bx + (p ^ 1), ((step - 1) >> 1) & 1, fail, a.spin);
                 own_of(K, lg, rank, f, cnt);
-                const bool dead = *fail;
-                if (cnt == 0 && !dead) send_credit(ycr + rank, by + p);
+                const bool mute = end || *fail;
+                if (cnt == 0 && !mute) send_credit(ycr + rank, by + p);
                 for (int o = o0; o - half < cnt; o += 2 * NC) {
                     if (o != o0) fetch_inv(cur, q, o);
                     T v[NR];
@@ -411,11 +412,11 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
                     mults_half<T, NR>(v, la, xs, K, tr ? f + o : 0, tr ? K : f + o + 1);
                     lane_sums<T, NR, 16>(v);
                     if (o < cnt) {
-                        if (!dead) send_all(y + (f + o) * NR + c, by + p, v[0]);
+                        if (!mute) send_all(y + (f + o) * NR + c, by + p, v[0]);
                         if (h % LC == 0 && c < nr) a.B[(cur.row0 + K0 + f + o) * a.ldb + c0 + c] = v[0];
                     }
                 }
-                if (last_block && last_q) break;
+                if (end) break;
                 // the next sub-block (of this block, or the first of the next one)
                 const Block<T>& nb = last_q ? nxt : cur;
                 const int nq = last_q ? (tr ? nxt.nsub - 1 : 0) : (tr ? q - 1 : q + 1);
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
                 const T* an = last_q ? acc_of(j + dj, ring, 1) : acc_of(j, ring, 0);
                 fetch_half<T>(l1, Mn + o0 * so, sk, o0 < on, K);
                 T* xn = xbuf + p * kBuf;
-                if (tid == 0) bar_expect(bx + p, xbytes(nb, nq));
+                if (tid == 0 && !*fail) bar_expect(bx + p, xbytes(nb, nq));
                 bar_wait(by + p, ph, fail, a.spin);
                 asm volatile("bar.sync %0, 384;" ::"r"(1 + (int)p) : "memory");  // the bulk update of the step before is done
                 // x of the next sub-block, own rows
@@ -602,10 +603,22 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
             ring = ring == 2 ? 0 : ring + 1;
         }
     }
-    // no CTA leaves while a peer may still store into it
+    // No CTA leaves while a peer may still store into it.  A cluster barrier does
+    // not cover st.async, whose completion shows on the receiver's mbarrier only;
+    // so every exchange that is sent is waited for by its receivers: each y by the
+    // chain's wait for it, each x by the next step's, and the last y is not sent.
+    // A CTA whose wait gave up has neither armed nor sent anything since.  What its
+    // peers sent it before they stopped (all have when the barrier below lets it
+    // pass) may be on its way to phases that never complete: it stays for 2^14
+    // polls of each barrier, some thousand times as long as a store takes.
     __syncthreads();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (*fail) {  // a wait gave up: the result is not one
+    if (*fail) {  // the result is not one
+        if (tid < 4) {
+            volatile int never = 0;
+            for (unsigned parity = 0; parity < 2; ++parity) bar_wait(bx + tid, parity, &never, 1 << 14);
+        }
+        __syncthreads();
         const int64_t N = a.n * a.b + a.a;
         for (int64_t e = tid; e < N * nr; e += NT) a.B[(e / nr) * a.ldb + c0 + e % nr] = T(NAN);
     }
