@@ -508,10 +508,14 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// A cluster barrier without memory ordering: the CTAs' last remote reads are done
-// (their values have been used), and the stores after them need not be waited for.
-__device__ __forceinline__ void cluster_sync_reads() {
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+// The same in two halves.  A CTA arrives when its remote reads are issued: the
+// release makes the arrival wait for every one of them, also for those whose
+// value nothing uses.  What it stores after the arrival is not waited for.
+__device__ __forceinline__ void cluster_arrive_reads() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait_reads() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Address of `local_addr` in the shared memory of CTA `rank` of this cluster.
@@ -706,7 +710,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         return P.transCin ? Ci[(int64_t)n * P.ldcin + m] : Ci[(int64_t)m * P.ldcin + n];
     };
     constexpr int kOwn = TC_BM / 2 * BN / TC_THREADS2;  // elements a thread writes in a K split, at most
-    double cpre[kOwn];
+    double cpre[kOwn], sum[kOwn];
     {
         const int nq = (TC_BM + ks - 1) / ks, r_lo = (int)rank * nq, nr = r_lo + nq <= TC_BM ? nq : TC_BM - r_lo;
 #pragma unroll
@@ -872,11 +876,18 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                             t += (long long)(((unsigned long long)__float_as_uint(part[h][q].w) << 32) |
                                              __float_as_uint(part[h][q].z));
                         }
-                        store(row, c, finish_exact(i0, t, eAs[row], eBs[c]), cpre[u0 + h]);
+                        sum[u0 + h] = finish_exact(i0, t, eAs[row], eBs[c]);
                     }
                 }
             }
-            cluster_sync_reads();
+            cluster_arrive_reads();
+            if (all_ok) {
+#pragma unroll
+                for (int u = 0; u < kOwn; ++u) {
+                    const int g = tid + u * TC_THREADS2;
+                    if (g < nr * BN) store(r_lo + g / BN, g % BN, sum[u], cpre[u]);
+                }
+            }
         } else {
         constexpr int LD2 = BN + 2;
         float2* R2 = (float2*)smem;
@@ -947,13 +958,24 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                     }
                     norm2(h0, l0);
                     norm2(h1, l1);
-                    store(row, c2, finish(h0, l0, eAs[row], eBs[c2]), cpre[2 * (u0 + h)]);
-                    store(row, c2 + 1, finish(h1, l1, eAs[row], eBs[c2 + 1]), cpre[2 * (u0 + h) + 1]);
+                    sum[2 * (u0 + h)] = finish(h0, l0, eAs[row], eBs[c2]);
+                    sum[2 * (u0 + h) + 1] = finish(h1, l1, eAs[row], eBs[c2 + 1]);
                 }
             }
         }
-        cluster_sync_reads();  // peers are done reading this CTA's accumulators
+        cluster_arrive_reads();
+        if (all_ok) {
+#pragma unroll
+            for (int u = 0; u < kOwn / 2; ++u) {
+                const int g = tid + u * TC_THREADS2;
+                if (g >= nr * G2) break;
+                const int row = r_lo + g / G2, c2 = (g % G2) * 2;
+                store(row, c2, sum[2 * u], cpre[2 * u]);
+                store(row, c2 + 1, sum[2 * u + 1], cpre[2 * u + 1]);
+            }
         }
+        }
+        cluster_wait_reads();  // peers are done reading this CTA's sums
     } else {
         // the whole K here: TMEM -> FP64 tile in shared memory -> coalesced writes
         double* Ds = (double*)smem;
