@@ -62,7 +62,11 @@ extern "C" {
 #define SGB_C128 3
 
 /* ---- precision modes ------------------------------------------------ */
-/* Arithmetic in the storage type throughout: the drop-in form. */
+/* Arithmetic in the storage type throughout: the drop-in form.  FP64 block
+ * products of pobtaf and pobtasi from b = 192 to 576 may be formed as sums of nine
+ * exact bf16 slice products, where these give an entry at least the digits of
+ * an FP64 sum, and as FP64 sums elsewhere; with a workspace of less than the
+ * queried size (down to what the FP64 sums need) all are FP64 sums. */
 #define SGB_PREC_NATIVE 0
 /* FP64 storage; the dense block products run on the tensor cores as exact
  * bf16 slice products (fixed-point split of each FP64 operand into S

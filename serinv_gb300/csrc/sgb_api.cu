@@ -77,19 +77,23 @@ int parse_inv_slices(int precision, int S) {
 
 // FP64 arithmetic of pobtaf's Schur products and of pobtasi on the tensor
 // cores: kExactSlices slices (63 bits below each row's largest entry, level
-// sums added as integers, one rounding to FP64 per element).  Against 64 bits
-// the selected inverse is 8.2e-16 .. 1.4e-15 off at n=32 b=512 a=64 where the
-// FP64 pipe's sums are 9.0e-16 .. 1.5e-15 off, the factor is the same, and with
-// rows and columns scaled by up to 10^+-6 neither changes (the products over
-// rows of an inverse are balanced by its diagonal).  The factorization of the
-// column blocks stays on the FP64 pipe.
-// Below the line the slicing and the longer epilogue cost more than the FP64
-// pipe's 16 x 16 tiles.  us, exact slices and FP64 pipe: selected inverse n=64
-// b=160 a=48 3299 / 3464 but a=0 3036 / 2554, b=176 a=16 3383 / 4103, b=208 3702 /
-// 4599, b=256 a=32 4125 / 8055, b=512 (n=32) 4600 / 26456; factorization n=64
-// b=160 a=0 5943 / 5632, b=176 a=16 6505 / 6703, b=192 a=64 6865 / 7160, b=240 8277
-// / 9164, b=512 (n=32) 10378 / 16960.
-constexpr int64_t kExactMin = 176;
+// sums added as integers, one rounding to FP64 per element), and the FP64 pipe
+// for elements whose terms are small beside the largest entries of their row and
+// column (sgb_gemm_tc.cu).  Every entry is as accurate as with FP64 sums, not the
+// norm alone.  Against 113 bits, n=2 b=256 a=32, relative error of an entry with
+// the slices and with the pipe, median and 99 %: selected inverse, diagonal blocks
+// 1.7e-16, 8.5e-16 and 3.4e-16, 1.9e-15, lower 2.1e-16, 1.0e-15 and 6.4e-16,
+// 3.2e-15; factor the same but for 1.70e-15 and 1.73e-15.  P = L^{-T} L^{-1} and the
+// factorization of the column blocks stay on the pipe.
+// Below the lines the slicing and the longer epilogue cost more than the FP64
+// pipe's 16 x 16 tiles.  ms, exact slices and FP64 pipe: factorization n=64 b=160
+// a=0 5.77 / 5.38, b=192 a=16 6.68 / 6.47, a=64 6.80 / 7.00, b=208 7.17 / 7.10, b=224
+// 7.50 / 7.71, b=256 a=32 8.43 / 9.59, b=512 a=64 20.7 / 31.3; selected inverse n=64
+// b=176 3.75 / 3.70, b=192 a=16 4.07 / 4.25, a=64 4.17 / 5.15, b=224 4.46 / 5.59,
+// b=512 a=64 13.2 / 53.4.  With fewer blocks the inversions ahead of the back-sweep
+// weigh more: n=24 b=208 1.63 / 1.58, b=224 1.64 / 2.00, n=6 b=208 0.49 / 0.42, b=224
+// 0.50 / 0.52.
+constexpr int64_t kExactMin = 224, kExactMinInv = 192;  // the latter from 32 blocks on
 
 // Whether a mixed factorization may take rows * L_ii^{-T} as a product: in place,
 // which only the tensor-core form does (it slices its operands first), and that
@@ -104,12 +108,10 @@ bool inverse_form(int64_t b) { return b > 2 * kTile && ceil_div(b, 32) * 32 <= k
 // and 5.4e-16 at b = 512.
 constexpr int64_t kPanelHalves = 416;
 
-// The slice count of a native FP64 sweep, or 0: the FP64 pipe.
-int exact_slices(const sgb_bta* m) {
-    return m->dtype == SGB_F64 && m->b >= kExactMin &&
-                   ceil_div(m->b, 32) * 32 <= kTcMaxK
-               ? kExactSlices
-               : 0;
+// The slice count of a native FP64 sweep (pobtaf, or pobtasi: inverse), or 0: the FP64 pipe.
+int exact_slices(const sgb_bta* m, bool inverse) {
+    const int64_t from = inverse && m->n >= 32 ? kExactMinInv : kExactMin;
+    return m->dtype == SGB_F64 && m->b >= from && ceil_div(m->b, 32) * 32 <= kTcMaxK ? kExactSlices : 0;
 }
 
 // Everything a block sweep needs besides the matrix: precision and the
@@ -127,7 +129,7 @@ struct Ctx {
 size_t tc_bound(int S, int64_t mx, int64_t kmax, int nprob) {
     const int64_t Mpad = ceil_div(mx, 128) * 128, Npad = ceil_div(mx, kTcBN) * kTcBN;
     const int64_t Kpad = ceil_div(kmax, 32) * 32 + 32;
-    const size_t per = (size_t)S * (Mpad + Npad) * Kpad * 2 + (size_t)(Mpad + Npad) * 4;
+    const size_t per = tc_inst_bytes(S, Mpad, Npad, Kpad);
     return (size_t)nprob * ((per + 255) / 256 * 256 + 256);
 }
 
@@ -220,7 +222,7 @@ size_t trtri_tc_bytes(int S, int64_t m, int64_t batch) {
         const int64_t pairs = (m / h + 1) / 2;
         const int64_t group = pairs < 4 ? pairs : 4;
         const int64_t Mpad = ceil_div(h, 128) * 128, Npad = ceil_div(h, kTcBN) * kTcBN, Kpad = ceil_div(h, 32) * 32;
-        const size_t per = (size_t)S * (Mpad + Npad) * Kpad * 2 + (size_t)(Mpad + Npad) * 4;
+        const size_t per = tc_inst_bytes(S, Mpad, Npad, Kpad);
         const size_t bytes = (size_t)group * ((size_t)batch * ((per + 255) / 256 * 256) + 256);
         best = bytes > best ? bytes : best;
     }
@@ -294,7 +296,7 @@ constexpr int64_t kSiTcBatch = 16;
 size_t tc_prob_bytes(int S, int64_t M, int64_t N, int64_t Kpad, int64_t batch) {
     const int64_t Mpad = ceil_div(M, 128) * 128, Npad = ceil_div(N, kTcBN) * kTcBN;
     const int64_t Kal = Kpad <= 0 ? 32 : ceil_div(Kpad, 32) * 32;
-    const size_t per = (size_t)S * (Mpad + Npad) * Kal * 2 + (size_t)(Mpad + Npad) * 4;
+    const size_t per = tc_inst_bytes(S, Mpad, Npad, Kal);
     return (per + 255) / 256 * 256 * (size_t)batch + 256;
 }
 
@@ -357,11 +359,11 @@ size_t tasi_bytes(const sgb_bta* m, int S, int Si, int64_t cap = kSiChunk) {
     return m->dtype == SGB_F64 ? PobtasiWs<double>(m, S, Si, cap).total : PobtasiWs<float>(m, S, Si, cap).total;
 }
 int taf_slices(const sgb_bta* m, int S, size_t have) {
-    const int X = S ? 0 : exact_slices(m);
+    const int X = S ? 0 : exact_slices(m, false);
     return X && have >= taf_bytes(m, X, 0) ? X : S;
 }
 int tasi_slices(const sgb_bta* m, int S, size_t have) {
-    const int X = S ? 0 : exact_slices(m);
+    const int X = S ? 0 : exact_slices(m, true);
     return X && have >= tasi_bytes(m, X, 0) ? X : S;
 }
 
@@ -950,7 +952,7 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
     cx.status = (int32_t*)(base + W.status);
     Ctx cxi = cx;  // the inversions and the products with L_ii^{-1}
     cxi.slices = Si ? Si : S;
-    Ctx cxt = cxi;  // the tip: too small for the exact slices to pay
+    Ctx cxt = cxi;  // without the exact slices: the tip, for which they do not pay, and P
     if (S > 7) cxt.slices = 0;
     T* Linv = (T*)(base + W.linv);
     T* Ltinv = (T*)(base + W.linv_tip);
@@ -1016,6 +1018,12 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 p.strideC = ghs;
                 pr[np++] = p;
             }
+            if (S > 7) {
+                // not P_j, whose entries off the diagonal are 2^-10 of it for a dominant
+                // matrix and would nearly all be summed on the FP64 pipe one by one
+                SGB_TRY(run_gemm<T>(cxi, pr, np, s));
+                np = 0;
+            }
             {  // P_j = L_jj^{-T} L_jj^{-1} into D_j
                 GemmProb<T> p = prob<T>();
                 p.M = p.N = (int32_t)b;
@@ -1026,9 +1034,11 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 p.Cout = B.d(j0);
                 p.ldc = b;
                 p.strideC = bb;
+                p.lower_only = S > 7;
                 pr[np++] = p;
             }
-            SGB_TRY(run_gemm<T>(cxi, pr, np, s));
+            SGB_TRY(run_gemm<T>(S > 7 ? cxt : cxi, pr, np, s));
+            if (S > 7) SGB_TRY(mirror_lower((double*)B.d(j0), b, bb, jn, s));  // (FP64 only)
         }
         for (int64_t i = hi - 1; i >= lo; --i) {
             const bool has_next = i < n - 1;
@@ -1679,7 +1689,7 @@ int plan_item(const sgb_bta* m, int ops, int precision, void* rhs, int64_t nrhs,
     sgb_pobtaf_workspace_size(m, precision, &need);
     if ((rc = check_ws(w, wb, need))) return rc;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
-    SGB_TRY(cudaMemsetAsync(w, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(w, 0, kStatusBytes, s));
     bool filled = false;
     const int Si = parse_inv_slices(precision, S);
     if ((rc = pobtaf_run<double>(m, 1, S, Si, w, info, s, nullptr, xall, &filled))) return rc;
@@ -1751,7 +1761,7 @@ int stream_sizes(const sgb_bta* host, int precision, int64_t ring, bool inverse,
     const int Si = parse_inv_slices(precision, S);
     *R = inverse ? ring_slots(ring, kRingPobtasi, true) : ring_slots(ring, kRingPobtaf, false);
     if (*R < 2 || *R > ((int64_t)1 << 20)) return SGB_ERR_SHAPE;
-    for (int X : {S ? S : exact_slices(host), S}) {
+    for (int X : {S ? S : exact_slices(host, inverse), S}) {
         *slices = X;
         *sweep = inverse ? tasi_bytes(host, X, Si, *R / 2) : taf_bytes(host, X, Si);
         *total = StreamWs(host, *sweep, *R).total;
@@ -1794,7 +1804,7 @@ int sgb_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes) {
     if (S < 0) return -S;
     if (!bytes) return SGB_ERR_ARG;
     const int Si = parse_inv_slices(precision, S);
-    *bytes = m->dtype == SGB_F64 ? PobtafWs<double>(m, S ? S : exact_slices(m), Si).total
+    *bytes = m->dtype == SGB_F64 ? PobtafWs<double>(m, S ? S : exact_slices(m, false), Si).total
                                  : PobtafWs<float>(m, S, Si).total;
     return SGB_OK;
 }
@@ -1807,7 +1817,7 @@ int sgb_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes) {
     if (S < 0) return -S;
     if (!bytes) return SGB_ERR_ARG;
     const int Si = parse_inv_slices(precision, S);
-    *bytes = m->dtype == SGB_F64 ? PobtasiWs<double>(m, S ? S : exact_slices(m), Si).total
+    *bytes = m->dtype == SGB_F64 ? PobtasiWs<double>(m, S ? S : exact_slices(m, true), Si).total
                                  : PobtasiWs<float>(m, S, Si).total;
     return SGB_OK;
 }
@@ -1904,7 +1914,7 @@ int sgb_pobtaf(const sgb_bta* m, int factorize_last_block, int precision, void* 
         return SGB_OK;
     }
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     if (m->dtype == SGB_F64)
         return pobtaf_run<double>(m, factorize_last_block, taf_slices(m, S, workspace_bytes), Si, workspace, info, s);
     return pobtaf_run<float>(m, factorize_last_block, S, Si, workspace, info, s);
@@ -1928,7 +1938,7 @@ int sgb_pobtasi(const sgb_bta* m, int invert_last_block, int precision, void* wo
                                     : small_inverse<float>(m, invert_last_block, status, s));
         return SGB_OK;
     }
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     if (m->dtype == SGB_F64)
         return pobtasi_run<double>(m, invert_last_block, tasi_slices(m, S, workspace_bytes), Si, workspace, s);
     return pobtasi_run<float>(m, invert_last_block, S, Si, workspace, s);
@@ -1974,7 +1984,7 @@ int sgb_pobtaf_permuted(const sgb_bta* m, void* buffer, int precision, void* wor
     if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     if (m->dtype == SGB_F64) return pobtaf_permuted_run<double>(m, (double*)buffer, S, Si, workspace, info, s);
     return pobtaf_permuted_run<float>(m, (float*)buffer, S, Si, workspace, info, s);
 }
@@ -2019,7 +2029,7 @@ int sgb_pobtasi_permuted(const sgb_bta* m, void* buffer, int precision, void* wo
     sgb_pobtasi_permuted_workspace_size(m, precision, &need);
     if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     if (m->dtype == SGB_F64) return pobtasi_permuted_run<double>(m, (double*)buffer, S, Si, workspace, s);
     return pobtasi_permuted_run<float>(m, (float*)buffer, S, Si, workspace, s);
 }
@@ -2114,7 +2124,7 @@ int sgb_pobtaf_host(const sgb_bta* host, const sgb_bta* dev, int factorize_last_
     if ((rc = check_ws(workspace, workspace_bytes, taf_bytes(dev, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     HostLink hl;
     hl.h = host;
     hl.d = dev;
@@ -2158,7 +2168,7 @@ int sgb_pobtaf_stream(const sgb_bta* host, int factorize_last_block, int precisi
     const sgb_bta dm = ring_desc(host, (char*)workspace, L);
     cudaStream_t s = (cudaStream_t)stream;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     HostRing hr;
     hr.h = host;
     hr.dD = (char*)dm.diag;
@@ -2187,7 +2197,7 @@ int sgb_pobtasi_stream(const sgb_bta* host, int invert_last_block, int precision
     const StreamWs L(host, sweep, R);
     const sgb_bta dm = ring_desc(host, (char*)workspace, L);
     cudaStream_t s = (cudaStream_t)stream;
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     HostRing hr;
     hr.h = host;
     hr.dD = (char*)dm.diag;
@@ -2212,7 +2222,7 @@ int sgb_pobtasi_host(const sgb_bta* host, const sgb_bta* dev, int invert_last_bl
     const int Si = parse_inv_slices(precision, S);
     if ((rc = check_ws(workspace, workspace_bytes, tasi_bytes(dev, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    SGB_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t), s));  // status word
+    SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));
     HostLink hl;
     hl.h = host;
     hl.d = dev;

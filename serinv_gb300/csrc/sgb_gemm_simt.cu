@@ -504,6 +504,20 @@ __global__ void __launch_bounds__(ST) k_gemm_small(const __grid_constant__ GemmL
     }
 }
 
+// Upper 32 x 32 tiles of `batch` m x m blocks from the lower ones, transposed.
+__global__ void __launch_bounds__(256) k_mirror(double* X, int64_t m, int64_t stride) {
+    __shared__ double t[32][33];
+    int i = 1, j = blockIdx.x;  // tile (i, j) below the diagonal: j of i, row after row
+    while (j >= i) j -= i++;
+    double* B = X + blockIdx.y * stride;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    for (int r = y; r < 32; r += 8)
+        if (i * 32 + r < m) t[r][x] = B[(int64_t)(i * 32 + r) * m + j * 32 + x];
+    __syncthreads();
+    for (int r = y; r < 32; r += 8)
+        if (i * 32 + x < m) B[(int64_t)(j * 32 + r) * m + i * 32 + x] = t[x][r];
+}
+
 template <typename T, int TM, int TN>
 cudaError_t launch_small(const GemmLaunch<T>& L, unsigned grid, cudaStream_t s) {
     cudaLaunchConfig_t cfg;
@@ -733,6 +747,15 @@ cudaError_t gemm_simt(GemmProb<T>* probs, int np, cudaStream_t s) {
     }
     prof_after(SGB_KCLASS_GEMM, s, fl);
     return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+cudaError_t mirror_lower(double* X, int64_t m, int64_t stride, int64_t batch, cudaStream_t s) {
+    const int64_t nt = ceil_div(m, 32);
+    if (nt < 2 || batch <= 0) return cudaSuccess;
+    prof_before(s, SGB_KCLASS_GEMM);
+    k_mirror<<<dim3((unsigned)(nt * (nt - 1) / 2), (unsigned)batch), 256, 0, s>>>(X, m, stride);
+    prof_after(SGB_KCLASS_GEMM, s, 0.0);
+    return cudaGetLastError();
 }
 
 template cudaError_t gemm_simt<double>(GemmProb<double>*, int, cudaStream_t);

@@ -28,6 +28,26 @@
 // inverse's columns and the rows they meet may differ by any factor, and a
 // fixed-point row keeps only what lies 63 bits below its largest entry.
 //
+// What that leaves out is of the size of 2^(EA + EB), EA and EB the exponents of
+// the row's and the column's largest entries, so an element whose own terms are
+// much smaller would have fewer digits than an FP64 sum gives it.  The MMAs
+// therefore also form N = sum |a||b| of every element, from one more slice of each
+// operand that holds the magnitudes as floating-point numbers, and an element with
+// 0 < N < kPipeBelow 2^(EA + EB) is summed on the FP64 pipe instead, as are those
+// of rows and columns that hold Infs, NaNs or subnormal numbers.  Error over
+// sum |a||b|, rms, K = 512, nine slices and FP64 pipe, by N 2^-(EA + EB): 2^-6
+// 2^-53.3 and 2^-53.5, 2^-5 2^-54.1 and 2^-53.4, 2^-4 2^-54.3 and 2^-53.0, from 2^-3
+// on 2^-54.2 or less and 2^-51.2 to 2^-52.5 (products with the inverse of a
+// dominant factor); flat operands 2^-58.3 and 2^-55.3.  Of the sweeps' products
+// with such matrices one element in 500 is below the line, with a decaying inverse
+// nearly all.  A warp sums single elements, 32 k at a time.  A CTA where these are
+// a quarter of the elements of most threads sums its whole part of the tile as FP64
+// tiles; and after a product in which most CTAs did, the slicing launches of the call's other products
+// form these so, spread over all SMs, instead of slicing.  ms, n=32, factorization
+// and selected inverse of matrices of decaying blocks, so and with the FP64 pipe's
+// own kernels: b=192 3.9, 3.2 and 3.2, 2.0; b=320 7.0, 8.9 and 6.6, 6.8; b=512 19.6,
+// 31.9 and 15.6, 26.3 (with single elements only 40, 156).
+//
 // This is the published Ozaki error-free splitting idea (Ozaki, Ogita,
 // Oishi, Rump) specialised to fixed-point digits and level-grouped exact
 // tensor-core accumulation.
@@ -105,8 +125,9 @@ struct SplitJob {
     __nv_bfloat16* out;   // per instance, A: [S][Rpad/RT][Kpad/32] chunks of RT x 32 (core-matrix order)
                           // [k/8][row/8][8][8]; B: [Rpad/RT][Kpad/32] chunks of S x RT x 32 in the order
                           // [k/8][slice][row/8][8][8], so that one MMA takes several slices side by side
+    int64_t mag;          // S = 9: elements from out to the magnitudes, [Rpad/RT][Kpad/32] chunks as A's slices
     int32_t* exps;        // [Rpad] per instance: kExpBias + biased FP64 exponent of the row max, 0 for a zero
-                          // row, kExpNan for a row that holds an Inf or NaN
+                          // row, kExpOdd for a row that holds an Inf or NaN (S = 9: or a subnormal number)
     int64_t out_stride, exp_stride;
     int32_t R, Rpad, Kpad;
     int32_t RT;           // rows per chunk: 128 for A, the tile width for B
@@ -116,24 +137,11 @@ struct SplitJob {
 };
 
 constexpr int kExpBias = 8192;  // keeps a scaled exponent positive
-constexpr int kExpNan = -1;
+constexpr int kExpOdd = -1;
+constexpr float kPipeBelow = 0x1p-5f;  // S = 9: elements below this share of 2^(EA + EB) go to the FP64 pipe
 constexpr int kSplitRows = 8;
 constexpr int kSplitThreads = 512;  // two CTAs per SM, eight warps per scheduler: latency bound
 constexpr int kSplitLd = kTcMaxK + 1;  // odd stride: conflict-free row and column access
-
-struct SplitLaunch {
-    SplitJob j[kMaxSplitJobs];
-    int32_t nj;
-    int32_t S;
-};
-
-__device__ __forceinline__ int find_job(const SplitLaunch& L, int cta) {
-    int ji = 0;
-#pragma unroll 1
-    for (int q = 1; q < L.nj; ++q)
-        if (cta >= L.j[q].strip_begin) ji = q;
-    return ji;
-}
 
 // Balanced base-128 digits of x 2^sk scaled by the row exponent Erow (biased).
 template <int S>
@@ -186,6 +194,55 @@ __device__ __forceinline__ void digits(double x, int sk, int Erow, int (&d)[S]) 
     d[0] = hi;
 }
 
+// |x| 2^sk in units of 2^Erow as a bf16 (truncated; at least 2^-60 unless zero, so
+// that no product of two underflows).  x is normal or zero.
+__device__ __forceinline__ uint32_t magnitude(double x, int sk, int Erow) {
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const int Ex = (int)((hi >> 20) & 0x7ff);
+    if (Ex == 0) return 0u;
+    const int e = Ex + sk - Erow;
+    return e < -60 ? (127u - 60u) << 7 : ((unsigned)(127 + e) << 7) | ((hi >> 13) & 0x7fu);
+}
+
+// Whether a product with nine slices runs on the FP64 pipe (StatusWord).  Its slicing
+// launch decides: it looks at what the product before it counted (all of its CTAs
+// find the same, whether or not the first of them has noted it already).
+struct PipeMode {
+    int32_t* words;  // the status slot
+    int32_t number;  // of the product; the ones of a call are numbered upwards
+    int32_t before;  // CTAs with elements of the product before it
+    __device__ __forceinline__ bool noted() const {
+        const int32_t f = ((const volatile int32_t*)words)[SW_PIPE];
+        return f != 0 && f <= number;
+    }
+    __device__ __forceinline__ bool decide() const {
+        const int32_t n = ((const volatile int32_t*)words)[SW_PARTS + ((number - 1) & 1)];
+        const bool pipe = noted() | (2 * n > before);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            words[SW_PARTS + (number & 1)] = 0;
+            if (pipe && words[SW_PIPE] == 0) words[SW_PIPE] = number;
+        }
+        return pipe;
+    }
+    __device__ __forceinline__ void count() const { atomicAdd(words + SW_PARTS + (number & 1), 1); }
+};
+
+struct SplitLaunch {
+    SplitJob j[kMaxSplitJobs];
+    int32_t nj;
+    int32_t S;
+    int32_t strips;  // of all jobs
+    PipeMode mode;
+};
+
+__device__ __forceinline__ int find_job(const SplitLaunch& L, int cta) {
+    int ji = 0;
+#pragma unroll 1
+    for (int q = 1; q < L.nj; ++q)
+        if (cta >= L.j[q].strip_begin) ji = q;
+    return ji;
+}
+
 // Programmatic dependent launch: the kernels of a product are launched
 // with programmatic stream serialization, so a launch may start while its
 // predecessor in the stream drains.  Every kernel waits for the
@@ -196,19 +253,157 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A term as the caller gave it, for the elements that the FP64 pipe sums.
+struct TcTerm {
+    const double* A;
+    const double* B;
+    int64_t lda, ldb, strideA, strideB;
+    int32_t K;
+    int8_t transA, transB, kmode;
+};
+
+struct TcProb {
+    const __nv_bfloat16* A;  // [S][Mpad][Kpad], then (S = 9) the magnitudes
+    const __nv_bfloat16* B;  // [S][Npad][Kpad], likewise
+    const int32_t* eA;
+    const int32_t* eB;
+    const double* Cin;
+    double* Cout;
+    int64_t strideA, strideB, strideEA, strideEB, strideCin, strideC;
+    int64_t ldcin, ldc;
+    double alpha, beta;
+    int32_t M, N, Mpad, Npad, Kpad;
+    int32_t batch;
+    int32_t lower_only, transCin;
+    int32_t tiles_m, tiles_n, tile_begin;
+    int32_t nterms;
+    TcTerm term[2];
+};
+
+// Element (m, n) of the terms' product on the FP64 pipe, one warp, k over the lanes.
+__device__ __noinline__ double pipe_sum(const TcProb& P, int inst, int m, int n) {
+    double s = 0.0;
+    for (int t = 0; t < P.nterms; ++t) {
+        const TcTerm& g = P.term[t];
+        const double* A = g.A + (int64_t)inst * g.strideA + (int64_t)m * (g.transA ? 1 : g.lda);
+        const double* B = g.B + (int64_t)inst * g.strideB + (int64_t)n * (g.transB ? g.ldb : 1);
+        const int64_t ak = g.transA ? g.lda : 1, bk = g.transB ? 1 : g.ldb;
+        const int lo = g.kmode == KM_GE_N0 ? n : g.kmode == KM_GE_M0 ? m : 0;
+        const int hi = g.kmode == KM_LT_N1 ? min(g.K, n + 1) : g.kmode == KM_LT_M1 ? min(g.K, m + 1) : g.K;
+#pragma unroll 4
+        for (int k = lo + (int)(threadIdx.x & 31); k < hi; k += 32) s = fma(A[k * ak], B[k * bk], s);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// Rows [m_lo, m_hi) and columns [n_lo, n_hi) of a product on the FP64 pipe by the
+// whole CTA of G x 256 threads, 16 x 16 elements at a time: every stride-th of these
+// tiles from the first-th on.  64 k are staged at a time, the next 64 on their way
+// meanwhile; thread group g sums every G-th of them.  Returns the number of tiles.
+struct PipeTile {
+    double a[64][17], b[64][17];
+};
+template <int G>
+__device__ __noinline__ int pipe_tiles(const TcProb& P, int inst, int m_lo, int m_hi, int n_lo, int n_hi, int first,
+                                       int stride, PipeTile& S) {
+    constexpr int U = 4 / G;  // elements of a slab that a thread stages, per operand
+    const int tid = threadIdx.x, grp = tid >> 8, r = (tid >> 4) & 15, c = tid & 15;
+    const int tn = (n_hi - n_lo + 15) / 16, tiles = (m_hi - m_lo + 15) / 16 * tn;
+    double* C = P.Cout + (int64_t)inst * P.strideC;
+    const double* Ci = P.Cin ? P.Cin + (int64_t)inst * P.strideCin : nullptr;
+    for (int i = first; i < tiles; i += stride) {
+        const int m0 = m_lo + i / tn * 16, n0 = n_lo + i % tn * 16, m1 = min(m0 + 16, m_hi), n1 = min(n0 + 16, n_hi);
+        if (P.lower_only && n0 >= m1) continue;
+        double acc = 0.0;
+        for (int t = 0; t < P.nterms; ++t) {
+            const TcTerm& g = P.term[t];
+            const double* A = g.A + (int64_t)inst * g.strideA;
+            const double* B = g.B + (int64_t)inst * g.strideB;
+            const int lo = g.kmode == KM_GE_N0 ? n0 : g.kmode == KM_GE_M0 ? m0 : 0;
+            const int hi = g.kmode == KM_LT_N1 ? min(g.K, n1) : g.kmode == KM_LT_M1 ? min(g.K, m1) : g.K;
+            double va[U], vb[U];
+            auto fetch = [&](int k0) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int e = tid + u * 256 * G, w = e / 64, k = e % 64;  // along k, or along the tile
+                    const int m = m0 + (g.transA ? e % 16 : w), ka = k0 + (g.transA ? e / 16 : k);
+                    const int n = n0 + (g.transB ? w : e % 16), kb = k0 + (g.transB ? k : e / 16);
+                    va[u] = m < m1 && ka < hi ? A[g.transA ? (int64_t)ka * g.lda + m : (int64_t)m * g.lda + ka] : 0.0;
+                    vb[u] = n < n1 && kb < hi ? B[g.transB ? (int64_t)n * g.ldb + kb : (int64_t)kb * g.ldb + n] : 0.0;
+                }
+            };
+            if (lo < hi) fetch(lo);
+            for (int k0 = lo; k0 < hi; k0 += 64) {
+                __syncthreads();  // the slab before is no longer read
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int e = tid + u * 256 * G, w = e / 64, k = e % 64;
+                    S.a[g.transA ? e / 16 : k][g.transA ? e % 16 : w] = va[u];
+                    S.b[g.transB ? k : e / 16][g.transB ? w : e % 16] = vb[u];
+                }
+                __syncthreads();
+                if (k0 + 64 < hi) fetch(k0 + 64);
+                const int kn = min(64, hi - k0);
+#pragma unroll 8
+                for (int k = grp; k < kn; k += G) acc = fma(S.a[k][r], S.b[k][c], acc);
+            }
+        }
+        if constexpr (G > 1) {  // the groups' sums
+            __syncthreads();
+            if (grp > 0) S.a[(grp - 1) * 16 + r][c] = acc;
+            __syncthreads();
+            if (grp > 0) continue;
+#pragma unroll
+            for (int q = 1; q < G; ++q) acc += S.a[(q - 1) * 16 + r][c];
+        }
+        const int m = m0 + r, n = n0 + c;
+        if (m >= m1 || n >= n1 || (P.lower_only && n > m)) continue;
+        double v = P.alpha * acc;
+        if (Ci != nullptr && P.beta != 0.0)
+            v = fma(P.beta, P.transCin ? Ci[(int64_t)n * P.ldcin + m] : Ci[(int64_t)m * P.ldcin + n], v);
+        C[(int64_t)m * P.ldc + n] = v;
+    }
+    return tiles;
+}
+
+// The problems of a product with nine slices, for its slicing launch.
+struct PipeProduct {
+    TcProb p[kMaxTcProbs];
+    int32_t np;
+};
+struct NoProduct {};
+
 // One CTA per strip of kSplitRows rows of one operand instance: the whole
 // strip (all terms, K <= kTcMaxK) is staged in shared memory with coalesced
 // loads, each row's largest exponent is found by one warp, and the S slices
 // of every element are written in the chunk layout the MMA descriptors
 // read -- padding rows and the K padding of each term as zeros, so the
 // buffers need no clearing beforehand.
-template <int S>
-__global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__ SplitLaunch L) {
+// With nine slices the launch forms the product itself when it is to run on the FP64
+// pipe: sixteen warps fill the pipe of an SM, and its grid may cover the SMs (the
+// CTAs past the strips have nothing else to do).
+template <int S, typename Product>
+__global__ void __launch_bounds__(kSplitThreads, S > 7 ? 1 : 2)
+    k_split(const __grid_constant__ SplitLaunch L, const __grid_constant__ Product W) {
     __shared__ double t[kSplitRows][kSplitLd];
+    static_assert(sizeof(t) >= sizeof(PipeTile), "one slab");
     __shared__ int ex[kSplitRows];
     constexpr bool kScaled = S > 7;
     __shared__ short sk[kScaled ? kTcMaxK : 1];  // power of two of each k
     pdl_enter();
+    if constexpr (kScaled) {
+        if (L.mode.decide()) {  // tiles of all problems, dealt to the CTAs in turn
+            const int ctas = (int)gridDim.x;
+            for (int q = 0, done = 0; q < W.np; ++q)
+                for (int i = 0; i < W.p[q].batch; ++i)
+                    done += pipe_tiles<kSplitThreads / 256>(W.p[q], i, 0, W.p[q].M, 0, W.p[q].N,
+                                                            ((int)blockIdx.x + ctas - done % ctas) % ctas, ctas, *(PipeTile*)t);
+            return;
+        }
+        if ((int)blockIdx.x >= L.strips) return;
+    }
     const SplitJob& J = L.j[find_job(L, blockIdx.x)];
     const int local = blockIdx.x - J.strip_begin;
     const int inst = local / J.strips;
@@ -279,9 +474,10 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
     if (warp < kSplitRows) {
         int emax = 0, bad = 0;
         for (int k = lane; k < J.Kpad; k += 32) {
-            int e = (int)(((unsigned long long)__double_as_longlong(t[warp][k]) >> 52) & 0x7ff);
+            const double x = t[warp][k];
+            int e = (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff);
             if constexpr (kScaled) {
-                bad |= e == 0x7ff;
+                bad |= e == 0x7ff || (e == 0 && x != 0.0);
                 if (e != 0) e += kExpBias + sk[k];
             }
             emax = e > emax ? e : emax;
@@ -295,7 +491,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
         }
         if (lane == 0) {
             ex[warp] = emax - kExpBias;  // not read for a zero row
-            J.exps[(int64_t)inst * J.exp_stride + r0 + warp] = bad ? kExpNan : emax;
+            J.exps[(int64_t)inst * J.exp_stride + r0 + warp] = bad ? kExpOdd : emax;
         }
     }
     __syncthreads();
@@ -313,12 +509,15 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
         const int rt = r / RT, ri = r % RT, kb = k0 >> 5, kk = k0 & 31;
         const int64_t o = ((int64_t)rt * nkb + kb) * (sd * RT * 32) + ((kk >> 3) * sd * (RT >> 3) + (ri >> 3)) * 64 +
                           (ri & 7) * 8;
-        uint32_t packed[S][4];
+        uint32_t packed[S][4], mag[4];
 #pragma unroll
         for (int j = 0; j < 8; j += 2) {
             int d0[S], d1[S];
-            digits<S>(t[rr][k0 + j], kScaled ? sk[k0 + j] : 0, ex[rr], d0);
-            digits<S>(t[rr][k0 + j + 1], kScaled ? sk[k0 + j + 1] : 0, ex[rr], d1);
+            const double x0 = t[rr][k0 + j], x1 = t[rr][k0 + j + 1];
+            const int s0 = kScaled ? sk[k0 + j] : 0, s1 = kScaled ? sk[k0 + j + 1] : 0;
+            digits<S>(x0, s0, ex[rr], d0);
+            digits<S>(x1, s1, ex[rr], d1);
+            mag[j >> 1] = kScaled ? magnitude(x0, s0, ex[rr]) | magnitude(x1, s1, ex[rr]) << 16 : 0u;
 #pragma unroll
             for (int p = 0; p < S; ++p) {
                 // w_p = d * 2^(-7p) is exact in bf16 (|d| <= 128)
@@ -330,26 +529,14 @@ __global__ void __launch_bounds__(kSplitThreads) k_split(const __grid_constant__
         for (int p = 0; p < S; ++p)
             *reinterpret_cast<uint4*>(out + p * slice + o) =
                 make_uint4(packed[p][0], packed[p][1], packed[p][2], packed[p][3]);
+        if constexpr (kScaled)
+            *reinterpret_cast<uint4*>(out + J.mag + ((int64_t)rt * nkb + kb) * (RT * 32) +
+                                      ((kk >> 3) * (RT >> 3) + (ri >> 3)) * 64 + (ri & 7) * 8) =
+                make_uint4(mag[0], mag[1], mag[2], mag[3]);
     }
 }
 
 // ---------------------------------------------------------------- tcgen05 GEMM
-
-struct TcProb {
-    const __nv_bfloat16* A;  // [S][Mpad][Kpad]
-    const __nv_bfloat16* B;  // [S][Npad][Kpad]
-    const int32_t* eA;
-    const int32_t* eB;
-    const double* Cin;
-    double* Cout;
-    int64_t strideA, strideB, strideEA, strideEB, strideCin, strideC;
-    int64_t ldcin, ldc;
-    double alpha, beta;
-    int32_t M, N, Mpad, Npad, Kpad;
-    int32_t batch;
-    int32_t lower_only, transCin;
-    int32_t tiles_m, tiles_n, tile_begin;
-};
 
 struct TcLaunch {
     TcProb p[kMaxTcProbs];
@@ -357,6 +544,7 @@ struct TcLaunch {
     int32_t ks;    // CTAs per output tile (a cluster), each over a K slice
     int32_t* err;  // set to SGB_ERR_TIMEOUT if a bounded wait gave up
     long long spin;  // poll limit of the pipeline's mbarrier waits
+    PipeMode mode;
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -527,8 +715,9 @@ __device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_addr, uint32_t ran
 
 template <int S, int BN>
 struct TcSmem {
-    static constexpr int kA = S * TC_BM * TC_BK * 2;   // bytes of A slices per stage
-    static constexpr int kB = S * BN * TC_BK * 2;      // bytes of B slices per stage
+    static constexpr int kA1 = TC_BM * TC_BK * 2, kB1 = BN * TC_BK * 2;  // bytes of one slice
+    static constexpr int kA = S * kA1;  // bytes of A slices per stage
+    static constexpr int kB = S * kB1;  // bytes of B slices per stage
     static constexpr int kStage = kA + kB;
     static constexpr int kBudget = 225 * 1024;
     static constexpr int kStages = (kBudget / kStage) > 4 ? 4 : (kBudget / kStage);
@@ -543,6 +732,7 @@ struct TcSmem {
     static constexpr int kBytes = kData + 1024 + 1024;
     static_assert(kBytes <= 227 * 1024, "shared memory per CTA");
     static_assert(kStages >= 2, "at least two pipeline stages");
+    static_assert(S <= 7 || kRed + (int)sizeof(PipeTile) <= kData, "FP64 tiles beside the sums");
 };
 
 // Warp roles (256 threads): warp 4 producer (bulk copies into a kStages
@@ -587,7 +777,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr bool kExact = S > 7;
     constexpr int NACC = S < 6 ? S : kExact ? 7 : 6;
-    constexpr int kUsed = NACC * BN;
+    constexpr int kUsed = (NACC + (kExact ? 1 : 0)) * BN;  // the levels, (S = 9) then N
     constexpr int kCols = kUsed <= 32 ? 32 : kUsed <= 64 ? 64 : kUsed <= 128 ? 128 : kUsed <= 256 ? 256 : 512;
     static_assert(kUsed <= 512, "TMEM columns");
 
@@ -612,6 +802,11 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     pdl_enter();
+    if (kExact && L.mode.noted()) {  // the slicing launch has formed the product
+        if (warp == 0)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+        return;
+    }
 
     const int nkb_all = P.Kpad / TC_BK;
     const int kb0 = (int)((int64_t)rank * nkb_all / ks), kb1 = (int)((int64_t)(rank + 1) * nkb_all / ks);
@@ -623,21 +818,33 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     const int64_t a_slice = (int64_t)P.Mpad * P.Kpad * 2;
     const int64_t a_tile = ((int64_t)mt * nkb_all + kb0) * (TC_BM * TC_BK * 2);
     const int64_t b_tile = ((int64_t)ntile * nkb_all + kb0) * SM::kB;
+    // ring rounds: first (S = 9) the magnitudes, S K blocks of them to a stage, then a K block's slices each
+    const int nmag = kExact ? (nkb + S - 1) / S : 0;
 
     if (warp == 4) {
         // producer
         if (lane == 0) {
             int issued = 0;
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int st = kb % NS, round = kb / NS;
-                if (kb >= NS && !mbar_wait(smem_u32(&empty[st]), (uint32_t)((round - 1) & 1), L.spin)) {
+            for (int it = 0; it < nmag + nkb; ++it) {
+                const int st = it % NS, round = it / NS, kb = it - nmag;
+                if (it >= NS && !mbar_wait(smem_u32(&empty[st]), (uint32_t)((round - 1) & 1), L.spin)) {
                     atomicExch(&flags[0], 1);
                     break;
                 }
-                issued = kb + 1;
+                issued = it + 1;
                 const uint32_t fb = smem_u32(&full[st]);
-                mbar_expect_tx(fb, (uint32_t)SM::kStage);
                 const uint32_t sA = sbase + st * SM::kStage, sB = sA + SM::kA;
+                if (kExact && kb < 0) {
+                    const int j0 = it * S, nj = nkb - j0 < S ? nkb - j0 : S;
+                    const uint32_t bytes = (uint32_t)nj * (SM::kA1 + SM::kB1);
+                    mbar_expect_tx(fb, bytes);
+                    bulk_g2s(sA, Ag + S * a_slice + a_tile + (int64_t)j0 * SM::kA1, nj * SM::kA1, fb);
+                    bulk_g2s(sB,
+                             Bg + (int64_t)S * P.Npad * P.Kpad * 2 + ((int64_t)ntile * nkb_all + kb0 + j0) * SM::kB1,
+                             nj * SM::kB1, fb);
+                    continue;
+                }
+                mbar_expect_tx(fb, (uint32_t)SM::kStage);
                 bulk_g2s(sB, Bg + b_tile + (int64_t)kb * SM::kB, SM::kB, fb);
 #pragma unroll 1
                 for (int p = 0; p < S; ++p)
@@ -659,14 +866,26 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
             // every accumulator, so it alone starts from zero.
             constexpr int kMaxQ = 256 / BN;
             constexpr uint32_t kGroup = S * (BN / 8) * 128;  // bytes from one 8-wide K group of B to the next
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int st = kb % NS, round = kb / NS;
+            for (int it = 0; it < nmag + nkb; ++it) {
+                const int st = it % NS, round = it / NS, kb = it - nmag;
                 if (!mbar_wait(smem_u32(&full[st]), (uint32_t)(round & 1), L.spin) || flags[0]) {
                     atomicExch(&flags[0], 1);
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t sA = sbase + st * SM::kStage, sB = sA + SM::kA;
+                if (kExact && kb < 0) {
+                    const int nj = nkb - it * S < S ? nkb - it * S : S;
+                    for (int j = 0; j < nj; ++j)
+#pragma unroll
+                        for (int ks = 0; ks < TC_BK / 16; ++ks)
+                            tc_mma(tmem + NACC * BN,
+                                   make_desc(sA + j * SM::kA1 + ks * 2 * (TC_BM / 8) * 128, (TC_BM / 8) * 128, 128),
+                                   make_desc(sB + j * SM::kB1 + ks * 2 * (BN / 8) * 128, (BN / 8) * 128, 128),
+                                   make_idesc(TC_BM, BN), it > 0 || j > 0 || ks > 0 ? 1u : 0u);
+                    tc_commit(smem_u32(&empty[st]));
+                    continue;
+                }
 #pragma unroll
                 for (int ks = 0; ks < TC_BK / 16; ++ks) {
 #pragma unroll
@@ -710,7 +929,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         return P.transCin ? Ci[(int64_t)n * P.ldcin + m] : Ci[(int64_t)m * P.ldcin + n];
     };
     constexpr int kOwn = TC_BM / 2 * BN / TC_THREADS2;  // elements a thread writes in a K split, at most
-    double cpre[kOwn], sum[kOwn];
+    double cpre[kOwn], sum[kOwn] = {};
     {
         const int nq = (TC_BM + ks - 1) / ks, r_lo = (int)rank * nq, nr = r_lo + nq <= TC_BM ? nq : TC_BM - r_lo;
 #pragma unroll
@@ -755,7 +974,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     // exponent 2047: its digits carry no value) makes the element NaN, as
     // the FP64 product would; a zero row or column otherwise gives 0
     auto finish = [&](float hi, float lo, int eAm, int eBn) -> double {
-        if (eAm == kExpNan || eBn == kExpNan) return __longlong_as_double(0x7ff8000000000000ll);
+        if (eAm == kExpOdd || eBn == kExpOdd) return __longlong_as_double(0x7ff8000000000000ll);
         if (eAm == 0 || eBn == 0) return 0.0;
         return scale_pow2(f32_to_f64(hi) + f32_to_f64(lo), eAm + eBn - 2058 - 2 * kExpBias);
     };
@@ -772,8 +991,13 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
             t += (long long)__float2int_rn(vv[6] * 0x1p45f);
         }
     };
-    auto finish_exact = [&](int i0, long long t, int eAm, int eBn) -> double {
-        if (eAm == kExpNan || eBn == kExpNan) return __longlong_as_double(0x7ff8000000000000ll);
+    // kToPipe: the element's terms are too small beside 2^(EA + EB), or its row or
+    // column holds numbers that have no digits
+    constexpr unsigned long long kToPipe = 0x7ff8000000000001ull;
+    auto to_pipe = [&](double r) { return (unsigned long long)__double_as_longlong(r) == kToPipe; };
+    auto finish_exact = [&](int i0, long long t, float mag, int eAm, int eBn) -> double {
+        if (eAm == kExpOdd || eBn == kExpOdd || (mag > 0.f && mag < kPipeBelow))
+            return __longlong_as_double((long long)kToPipe);
         if (eAm == 0 || eBn == 0) return 0.0;
         const long long hi = (long long)i0 + (t >> 45), lo = t & ((1ll << 45) - 1);
         return scale_pow2(fma(int_to_f64(hi), 0x1p45, int_to_f64(lo)), eAm + eBn - 2058 - 45 - 2 * kExpBias);
@@ -783,7 +1007,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
             int i0;
             long long t;
             fold(vv, i0, t);
-            return finish_exact(i0, t, eAm, eBn);
+            return finish_exact(i0, t, 0.f, eAm, eBn);  // N is looked at after it
         }
         float hi = vv[0], lo = 0.f;
 #pragma unroll
@@ -801,6 +1025,25 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
         else if (neg) r = -r;
         if (add_c) r = fma(P.beta, cv, r);
         C[(int64_t)m * P.ldc + n] = r;
+    };
+    // S = 9: the elements (row, col) that lanes of this warp hold in r and that go to
+    // the FP64 pipe, one after another by the whole warp
+    auto pipe_fill = [&](int row, int col, double& r) {
+        unsigned todo = __ballot_sync(0xffffffffu, to_pipe(r) && live(m0 + row, n0 + col));
+        while (todo) {
+            const int src = __ffs((int)todo) - 1;
+            todo &= todo - 1;
+            const double v = pipe_sum(P, inst, m0 + __shfl_sync(0xffffffffu, row, src), n0 + __shfl_sync(0xffffffffu, col, src));
+            if (lane == src) r = v;
+        }
+    };
+    // S = 9: the CTA's part, rows [r_lo, r_hi) of the tile, as FP64 tiles where most
+    // threads hold that many elements for the pipe
+    auto all_on_pipe = [&](bool many, int r_lo, int r_hi) {
+        if (__syncthreads_count(many) <= TC_THREADS2 / 2) return false;
+        if (tid == 0) L.mode.count();
+        pipe_tiles<1>(P, inst, m0 + r_lo, min(m0 + r_hi, P.M), n0, min(n0 + BN, P.N), 0, 1, *(PipeTile*)(smem + SM::kRed));
+        return true;
     };
     if (ks > 1) {
         // K split over the cluster: each CTA folds its level accumulators of
@@ -840,6 +1083,13 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                         fold(vv, i0, t);
                         RX[row * LDX + c0 + i] = make_int4(i0, 0, (int)t, (int)(t >> 32));
                     }
+                    if (nkb > 0) {  // N in the second word
+                        float mag[16];
+                        tmem_ld16_async(tmem + ((uint32_t)(q4 * 32) << 16) + NACC * BN + c0, mag);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) RX[row * LDX + c0 + i].y = __float_as_int(mag[i]);
+                    }
                 }
             }
             cluster_sync_all();
@@ -870,22 +1120,30 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                         const int row = r_lo + g / BN, c = g % BN;
                         int i0 = 0;
                         long long t = 0;
+                        float mag = 0.f;
 #pragma unroll
                         for (int q = 0; q < kTcMaxSplit; ++q) {
                             i0 += __float_as_int(part[h][q].x);
+                            mag += part[h][q].y;
                             t += (long long)(((unsigned long long)__float_as_uint(part[h][q].w) << 32) |
                                              __float_as_uint(part[h][q].z));
                         }
-                        sum[u0 + h] = finish_exact(i0, t, eAs[row], eBs[c]);
+                        sum[u0 + h] = finish_exact(i0, t, mag, eAs[row], eBs[c]);
                     }
                 }
             }
             cluster_arrive_reads();
             if (all_ok) {
+                int odd = 0;
+#pragma unroll
+                for (int u = 0; u < kOwn; ++u) odd += to_pipe(sum[u]);
+                const bool summed = all_on_pipe(odd * 4 * TC_THREADS2 > nr * BN, r_lo, r_lo + nr);
 #pragma unroll
                 for (int u = 0; u < kOwn; ++u) {
                     const int g = tid + u * TC_THREADS2;
-                    if (g < nr * BN) store(r_lo + g / BN, g % BN, sum[u], cpre[u]);
+                    if (summed || g >= nr * BN) break;  // (by whole warps)
+                    pipe_fill(r_lo + g / BN, g % BN, sum[u]);
+                    store(r_lo + g / BN, g % BN, sum[u], cpre[u]);
                 }
             }
         } else {
@@ -979,6 +1237,7 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     } else {
         // the whole K here: TMEM -> FP64 tile in shared memory -> coalesced writes
         double* Ds = (double*)smem;
+        int odd = 0;
         if (all_ok) {
             // as above: all eight warps, two column halves
             const int q4 = warp & 3, half = warp >> 2;
@@ -1002,10 +1261,23 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
                     for (int l = 0; l < NACC; ++l) vv[l] = v[l][i];
                     Ds[row * (BN + 1) + c0 + i] = combine(vv, eAm, eBs[c0 + i]);
                 }
+                if (kExact && nkb > 0) {
+                    float mag[16];
+                    tmem_ld16_async(tmem + ((uint32_t)(q4 * 32) << 16) + NACC * BN + c0, mag);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (mag[i] > 0.f && mag[i] < kPipeBelow) {
+                            Ds[row * (BN + 1) + c0 + i] = __longlong_as_double((long long)kToPipe);
+                            ++odd;
+                        }
+                }
             }
         }
         __syncthreads();
-        if (all_ok) {
+        bool summed = false;
+        if (kExact && all_ok) summed = all_on_pipe(odd * 4 * TC_THREADS2 > TC_BM * BN, 0, TC_BM);
+        if (all_ok && !summed) {
 #pragma unroll 1
             for (int e0 = tid; e0 < TC_BM * BN; e0 += 8 * TC_THREADS2) {
                 double cv[8];
@@ -1017,7 +1289,9 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int e = e0 + u * TC_THREADS2, row = e / BN, col = e % BN;
-                    store(row, col, Ds[row * (BN + 1) + col], cv[u]);
+                    double r = Ds[row * (BN + 1) + col];
+                    if constexpr (kExact) pipe_fill(row, col, r);
+                    store(row, col, r, cv[u]);
                 }
             }
         }
@@ -1069,8 +1343,8 @@ cudaError_t launch_tc(TcLaunch& L, int total_tiles, cudaStream_t s) {
     return cudaLaunchKernelEx(&cfg, k_gemm_tc<S, BN>, L);
 }
 
-template <int S>
-cudaError_t launch_split(const SplitLaunch& SL, int ctas, cudaStream_t s) {
+template <int S, typename Product = NoProduct>
+cudaError_t launch_split(const SplitLaunch& SL, int ctas, cudaStream_t s, const Product& W = Product()) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)ctas);
@@ -1082,7 +1356,7 @@ cudaError_t launch_split(const SplitLaunch& SL, int ctas, cudaStream_t s) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_split<S>, SL);
+    return cudaLaunchKernelEx(&cfg, k_split<S, Product>, SL, W);
 }
 
 // Whether two jobs slice the same numbers into the same layout.
@@ -1134,7 +1408,7 @@ size_t tc_workspace_bytes(const GemmProb<double>* probs, int np, int S) {
         if (Kpad == 0) Kpad = TC_BK;
         const int64_t Mpad = ceil_div(p.M, TC_BM) * TC_BM;
         const int64_t Npad = ceil_div(p.N, kTcBN) * kTcBN;
-        const size_t per = (size_t)S * (Mpad + Npad) * Kpad * 2 + (size_t)(Mpad + Npad) * 4;
+        const size_t per = tc_inst_bytes(S, Mpad, Npad, Kpad);
         total += (per * p.batch + 255) / 256 * 256 + 256;
     }
     return total;
@@ -1151,6 +1425,13 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
     SL.S = S;
     TcLaunch TL;
     memset(&TL, 0, sizeof(TL));
+    if (S > 7 && err == nullptr) return cudaErrorInvalidValue;
+    thread_local int32_t launches = 0;  // (a call's launches come from one host thread)
+    thread_local int32_t before = 0;
+    launches = launches == INT32_MAX - 1 ? 1 : launches + 1;  // odd and even in turn
+    SL.mode.before = TL.mode.before = before;
+    SL.mode.words = TL.mode.words = err;
+    SL.mode.number = TL.mode.number = launches;
     TL.err = err;
     TL.spin = spin_limit();
     char* base = (char*)ws;
@@ -1202,8 +1483,8 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         if (Kpad > kTcMaxK) return cudaErrorInvalidValue;
         const int64_t Mpad = ceil_div(p.M, TC_BM) * TC_BM;
         const int64_t Npad = ceil_div(p.N, kTcBN) * kTcBN;
-        const size_t bytesA = (size_t)S * Mpad * Kalloc * 2, bytesB = (size_t)S * Npad * Kalloc * 2;
-        const size_t per = bytesA + bytesB + (size_t)(Mpad + Npad) * 4;
+        const size_t bytesA = tc_planes(S) * Mpad * Kalloc * 2, bytesB = tc_planes(S) * Npad * Kalloc * 2;
+        const size_t per = tc_inst_bytes(S, Mpad, Npad, Kalloc);
         const size_t per_al = (per + 255) / 256 * 256;
         if (off + per_al * p.batch + 256 > ws_bytes) return cudaErrorInvalidValue;
         __nv_bfloat16* As = (__nv_bfloat16*)(base + off);
@@ -1253,6 +1534,7 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         ja.Kpad = (int32_t)Kalloc;
         ja.batch = p.batch;
         ja.strips = (int32_t)(Mpad / kSplitRows);
+        ja.mag = (int64_t)S * Mpad * Kalloc;
         jb.out = Bs;
         jb.exps = eB;
         jb.out_stride = ja.out_stride;
@@ -1264,6 +1546,7 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         jb.Kpad = (int32_t)Kalloc;
         jb.batch = p.batch;
         jb.strips = (int32_t)(Npad / kSplitRows);
+        jb.mag = (int64_t)S * Npad * Kalloc;
         // an operand that an earlier problem of the launch has too is sliced once
         for (SplitJob* j : {&ja, &jb}) {
             const SplitJob* same = nullptr;
@@ -1306,6 +1589,12 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
         tp.Kpad = (int32_t)Kpad;
         tp.batch = p.batch;
         tp.lower_only = p.lower_only;
+        for (int t = 0; t < p.nterms; ++t) {
+            const GemmTerm<double>& tm = p.term[t];
+            if (tm.K <= 0) continue;
+            TcTerm& g = tp.term[tp.nterms++];
+            g = {tm.A, tm.B, tm.lda, tm.ldb, tm.strideA, tm.strideB, tm.K, tm.transA, tm.transB, tm.kmode};
+        }
         tp.transCin = p.transCin;
         tp.tiles_m = (int32_t)(Mpad / TC_BM);
         tp.tiles_n = (int32_t)(Npad / bn);
@@ -1324,7 +1613,15 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
             case 5: e = launch_split<5>(SL, (int)split_ctas, s); break;
             case 6: e = launch_split<6>(SL, (int)split_ctas, s); break;
             case 7: e = launch_split<7>(SL, (int)split_ctas, s); break;
-            default: e = launch_split<kExactSlices>(SL, (int)split_ctas, s); break;
+            default: {
+                PipeProduct W;
+                memset(&W, 0, sizeof(W));
+                memcpy(W.p, TL.p, sizeof(W.p));
+                W.np = TL.np;
+                SL.strips = (int32_t)split_ctas;
+                e = launch_split<kExactSlices>(SL, shared_gpu || split_ctas > kTcSmCount ? (int)split_ctas : (int)kTcSmCount,
+                                               s, W);
+            }
         }
         prof_after(SGB_KCLASS_SPLIT, s, 0.0);
         if (e != cudaSuccess) return e;
@@ -1342,6 +1639,19 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
             for (int nt = 0; nt < tp.tiles_n; ++nt)
                 if (!(tp.lower_only && nt * bn >= mt * TC_BM + TC_BM)) ++run;
         issued += 2.0 * run * tp.batch * (double)TC_BM * bn * tp.Kpad * (S * (S + 1) / 2);
+    }
+    if (S > 7) {
+        before = 0;
+        for (int i = 0; i < TL.np; ++i) {
+            const TcProb& tp = TL.p[i];
+            const int rows = (TC_BM + ks - 1) / ks;
+            for (int m0 = 0; m0 < tp.M; m0 += TC_BM)
+                for (int m = m0; m < m0 + TC_BM && m < tp.M; m += rows) {
+                    const int end = m + rows < m0 + TC_BM ? m + rows : m0 + TC_BM;
+                    const int n_end = tp.lower_only && end < tp.N ? end : tp.N;
+                    before += (n_end + bn - 1) / bn * tp.batch;
+                }
+        }
     }
     cudaError_t e = tc_prepare();
     if (e != cudaSuccess) return e;

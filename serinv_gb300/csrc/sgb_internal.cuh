@@ -149,6 +149,10 @@ int capture_panel_grid();
 void set_capture_tc_split(bool on);
 bool capture_tc_split();
 
+// The tiles above the diagonal of `batch` m x m blocks that a lower_only product
+// left out, from those below (ld m).
+cudaError_t mirror_lower(double* X, int64_t m, int64_t stride, int64_t batch, cudaStream_t s);
+
 // Full triangular inverse of `batch` lower-triangular m x m blocks:
 // Linv_j = L_j^{-1} (zeros above the diagonal).  Scratch: batch*m*m T.
 // The row-sweep products go through `fn(fnctx, ...)` when given, else the
@@ -202,6 +206,18 @@ constexpr int kTcMaxK = 576;
 // Slice count of the products that stand in for FP64 arithmetic: 63 bits below
 // the row maxima, level sums added as integers (sgb_gemm_tc.cu).
 constexpr int kExactSlices = 9;
+// Planes of a sliced operand: its slices, and with kExactSlices the magnitudes.
+inline size_t tc_planes(int S) { return (size_t)(S > 7 ? S + 1 : S); }
+// Scratch of one instance of a product: both operands' planes, a word per row and column.
+inline size_t tc_inst_bytes(int S, int64_t Mpad, int64_t Npad, int64_t Kpad) {
+    return tc_planes(S) * (size_t)((Mpad + Npad) * Kpad * 2) + (size_t)(Mpad + Npad) * 4;
+}
+// Words of the status slot, zeroed when a call starts: the status, the caller's info,
+// and for products with kExactSlices the number of the first product of the call that
+// runs on the FP64 pipe (0: none), then for the last even and the last odd product the
+// CTAs that summed their part on the pipe.
+enum StatusWord { SW_STATUS = 0, SW_INFO = 1, SW_PIPE = 2, SW_PARTS = 3 };
+constexpr size_t kStatusBytes = 5 * sizeof(int32_t);
 size_t tc_workspace_bytes(const GemmProb<double>* probs, int np, int S);
 // Sets the tensor-core kernels' shared-memory attribute on the current
 // device (once); call before capturing launches into a graph.
