@@ -82,10 +82,14 @@ extern "C" {
  * times L_ii^{-T}, pobtasi's batched inversions and its products with
  * L_ii^{-1}: SGB_PREC_MIXED | (S << 8) | (Si << 16).  Any explicit Si takes
  * the inverse-based TRSMs, so S = Si = 7 is 7 slices everywhere at nearly
- * the 6-slice speed.
- * The first 4 bytes of the workspace receive a device status word (0, or
- * SGB_ERR_TIMEOUT if a bounded tensor-core wait gave up).                 */
+ * the 6-slice speed. */
 #define SGB_PREC_MIXED  1
+
+/* Device status: in either precision the first 4 bytes of the workspace of
+ * sgb_pobtaf, sgb_pobtasi, sgb_pobtas and their forms below receive a status word:
+ * 0, or SGB_ERR_TIMEOUT if a bounded device wait of the call gave up.  The call
+ * itself has returned by then.  What it was computing is not a result; right-hand
+ * sides of sgb_pobtas are NaN then. */
 
 typedef struct sgb_bta {
     int32_t dtype;     /* SGB_F32, SGB_F64, SGB_C64 or SGB_C128    */
@@ -143,6 +147,9 @@ int sgb_pobtaf(const sgb_bta* m, int factorize_last_block, int precision,
  */
 int sgb_pobtasi(const sgb_bta* m, int invert_last_block, int precision,
                 void* workspace, size_t workspace_bytes, void* stream);
+/* 1 if sgb_pobtasi with these sizes, this precision and a workspace of the queried
+ * size has bounded device waits, so that its status word is worth reading. */
+int sgb_pobtasi_has_waits(const sgb_bta* m, int precision);
 
 /*
  * In-place block triangular solve with the factor of sgb_pobtaf.
@@ -203,8 +210,7 @@ int sgb_pobtasi_stream(const sgb_bta* host, int invert_last_block, int precision
  * SGB_PREC_MIXED (FP64 storage) runs pobtaf's diagonal blocks through the
  * column-block kernel with L_ii^{-T} and every block product on the tensor
  * cores, and pobtasi's products likewise; the solve runs in the storage
- * precision in either mode, as sgb_pobtas does.  The first 4 bytes of the
- * pobtaf / pobtasi workspace receive the device status word.
+ * precision in either mode, as sgb_pobtas does.
  *
  * sgb_pobtaf_permuted: pobtaf(..., buffer=) (src/serinv/algs/pobtaf.py:
  *   58-76, _pobtaf_permuted :186-281).  Workspace:

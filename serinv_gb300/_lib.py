@@ -87,6 +87,7 @@ _SIGNATURES = {
                                   ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p]),
     "sgb_pobtasi": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_int, ctypes.c_int, ctypes.c_void_p,
                                    ctypes.c_size_t, ctypes.c_void_p]),
+    "sgb_pobtasi_has_waits": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_int]),
     "sgb_pobtas": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                   ctypes.c_char, ctypes.c_int, ctypes.c_int, ctypes.c_void_p,
                                   ctypes.c_size_t, ctypes.c_void_p]),

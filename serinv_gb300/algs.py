@@ -35,7 +35,9 @@ inverse, whose error grows with the conditioning); ``check_spd`` (pobtaf,
 default True) — synchronise and raise ``numpy.linalg.LinAlgError`` on a
 non-positive pivot, like SciPy's ``cholesky`` in the reference, and raise
 on a device wait that timed out (with False neither is checked and the call
-does not synchronise); ``ring_blocks`` (with ``device_streaming``) — blocks
+does not synchronise; pobtasi takes it for the device waits of its tensor-core
+products, default True; pobtas synchronises on device arrays only if given
+``check_spd=True``: after a wait that timed out ``B`` is NaN); ``ring_blocks`` (with ``device_streaming``) — blocks
 held on the device (default 4 for pobtaf, 32 for pobtasi).
 """
 
@@ -196,12 +198,14 @@ def _prepare(arrays, names):
     return device, wrapped
 
 
-def _finish(wrapped) -> None:
+def _finish(wrapped) -> bool:
+    """Host arrays get their results; True if there were any (the call has synchronised then)."""
     host = any(w.kind in ("numpy", "torch_host") for w in wrapped)
     for w in wrapped:
         w.writeback()
     if host:
         torch.cuda.current_stream(wrapped[0].t.device).synchronize()
+    return host
 
 
 def _pinned_host_stacks(arrays):
@@ -409,14 +413,14 @@ def pobtasi(L_diagonal_blocks, L_lower_diagonal_blocks, L_lower_arrow_blocks, L_
                                  precision, invert_last_block, kwargs.get("ring_blocks", 0), False)
             for t, x in back:
                 _copy_back(t, x)
-            _check_status(ws, precision, "pobtasi")
+            _check_status(ws, precision, "pobtasi", always=True)
             return
     host = _pinned_host_stacks(arrays)
     if host is not None:
         lib = _lib.load()
         ws, _ = _host_call(lib.sgb_pobtasi_host, lib.sgb_pobtasi_workspace_size, host, "pobtasi", precision,
                            invert_last_block, False)
-        _check_status(ws, precision, "pobtasi")
+        _check_status(ws, precision, "pobtasi", always=True)
         return
 
     lib = _lib.load()
@@ -432,8 +436,10 @@ def pobtasi(L_diagonal_blocks, L_lower_diagonal_blocks, L_lower_arrow_blocks, L_
         rc = lib.sgb_pobtasi(ctypes.byref(m), int(invert_last_block), precision, ws.data_ptr(), nbytes.value,
                              _stream(device))
         _lib.raise_for(rc, "pobtasi")
+        waits = lib.sgb_pobtasi_has_waits(ctypes.byref(m), precision) and bool(kwargs.get("check_spd", True)) \
+            and not torch.cuda.is_current_stream_capturing()
         _finish(w)
-        _check_status(ws, precision, "pobtasi")
+        _check_status(ws, precision, "pobtasi", always=waits)
 
 
 def pobtas(L_diagonal_blocks, L_lower_diagonal_blocks, L_lower_arrow_blocks, L_arrow_tip_block, B, trans="N",
@@ -485,7 +491,8 @@ def pobtas(L_diagonal_blocks, L_lower_diagonal_blocks, L_lower_arrow_blocks, L_a
         rc = lib.sgb_pobtas(ctypes.byref(m), _ptr(Bt), nrhs, max(nrhs, 1), trans.encode(), int(partial),
                             precision, ws.data_ptr(), nbytes.value, _stream(device))
         _lib.raise_for(rc, "pobtas")
-        _finish(w)
+        if _finish(w) or kwargs.get("check_spd", False):
+            _check_status(ws, precision, "pobtas", always=True)
 
 
 # --------------------------------------------------------------------------

@@ -336,14 +336,15 @@ struct PobtasiWs {
 
 template <typename T>
 struct PobtasWs {
-    size_t linv, linv_tip, trtri, y, total;
+    size_t trtri, linv, linv_tip, y, total;
     PobtasWs(const sgb_bta* m, int64_t nrhs) {
         const size_t n = m->n, b = m->b, a = m->a;
         const size_t mx = b > a ? b : a;
         Carve c;
+        // first, and free once the inverses exist: its first word is then the status
+        trtri = c.take(sizeof(T) * trtri_scratch_elems((int64_t)mx, (int64_t)n));
         linv = c.take(sizeof(T) * n * b * b);
         linv_tip = c.take(sizeof(T) * a * a);
-        trtri = c.take(sizeof(T) * trtri_scratch_elems((int64_t)mx, (int64_t)n));
         y = c.take(sizeof(T) * mx * (size_t)nrhs);
         total = c.off;
     }
@@ -1134,9 +1135,14 @@ int pobtas_native(const sgb_bta* m, T* Bm, int64_t nrhs, int64_t ldb, char trans
     T* Btip = Bm + n * b * ldb;
     auto Bi = [&](int64_t i) { return Bm + i * b * ldb; };
 
-    if (nrhs == 0) return SGB_OK;
+    // the status word of this call and of those that follow on the same inverses
+    int32_t* status = (int32_t*)(base + W.trtri);
+    if (nrhs == 0) {
+        SGB_TRY(cudaMemsetAsync(status, 0, sizeof(int32_t), s));
+        return SGB_OK;
+    }
     if (!partial && small_solve_ok<T>(m, nrhs)) {
-        SGB_TRY(small_solve<T>(m, Bm, nrhs, ldb, trans != 'N', s));
+        SGB_TRY(small_solve<T>(m, Bm, nrhs, ldb, trans != 'N', status, s));
         return SGB_OK;
     }
     Ctx native;
@@ -1151,11 +1157,12 @@ int pobtas_native(const sgb_bta* m, T* Bm, int64_t nrhs, int64_t ldb, char trans
         // with xall the block inverses exist already, as L_ii^{-T} (read transposed)
         if (!xall) SGB_TRY(trtri_run<T>(native, D, b, n, Linv, trs, s, sub));
         if (a && !partial) SGB_TRY(trtri_run<T>(native, Tp, a, 1, Ltinv, trs, s, sub));
+        SGB_TRY(cudaMemsetAsync(status, 0, sizeof(int32_t), s));
     }
     const T* Li = xall ? xall : Linv;
     const int tl = xall ? 1 : 0;
     if (chain) {
-        SGB_TRY(solve_chain<T>(m, Bm, nrhs, ldb, trans != 'N', Li, xall != nullptr, Ltinv, s));
+        SGB_TRY(solve_chain<T>(m, Bm, nrhs, ldb, trans != 'N', Li, xall != nullptr, Ltinv, status, s));
         return SGB_OK;
     }
 
@@ -1531,9 +1538,10 @@ int pobtas_permuted_run(const sgb_bta* m, T* buf, T* Bm, int64_t nrhs, int64_t l
     const int64_t bb = b * b, ab = a * b;
     T* Btip = Bm + n * b * ldb;
     auto Bi = [&](int64_t i) { return Bm + i * b * ldb; };
-    if (nrhs == 0 || n < 3) return SGB_OK;
     Ctx native;
-    SGB_TRY(trtri_run<T>(native, D + bb, b, n - 2, Linv, trs, s));  // blocks 1 .. n-2
+    if (nrhs > 0 && n >= 3) SGB_TRY(trtri_run<T>(native, D + bb, b, n - 2, Linv, trs, s));  // blocks 1 .. n-2
+    SGB_TRY(cudaMemsetAsync(base + W.trtri, 0, sizeof(int32_t), s));  // status word: no waits here
+    if (nrhs == 0 || n < 3) return SGB_OK;
     auto Li = [&](int64_t i) { return Linv + (i - 1) * bb; };
     if (trans == 'N') {  // pobtas.py:179-203
         for (int64_t i = 1; i < n - 1; ++i) {
@@ -1918,6 +1926,17 @@ int sgb_pobtaf(const sgb_bta* m, int factorize_last_block, int precision, void* 
     if (m->dtype == SGB_F64)
         return pobtaf_run<double>(m, factorize_last_block, taf_slices(m, S, workspace_bytes), Si, workspace, info, s);
     return pobtaf_run<float>(m, factorize_last_block, S, Si, workspace, info, s);
+}
+
+int sgb_pobtasi_has_waits(const sgb_bta* m, int precision) {
+    if (m == nullptr) return 0;
+    sgb_bta r = *m;
+    if (cx_dtype(m)) {
+        r.dtype = m->dtype == SGB_C128 ? SGB_F64 : SGB_F32;
+        r.b = 2 * m->b;
+    }
+    const int S = parse_precision(precision, r.dtype);
+    return S > 0 || (S == 0 && exact_slices(&r, true) > 0) ? 1 : 0;
 }
 
 int sgb_pobtasi(const sgb_bta* m, int invert_last_block, int precision, void* workspace, size_t workspace_bytes,

@@ -176,23 +176,26 @@ bool small_inverse_ok(const sgb_bta* m);
 template <typename T>
 cudaError_t small_inverse(const sgb_bta* m, int last, int32_t* status, cudaStream_t s);
 
-// One sweep of pobtas of small blocks in one launch, from the factor alone.
+// One sweep of pobtas of small blocks in one launch, from the factor alone; sets
+// *status to 0.
 template <typename T>
 bool small_solve_ok(const sgb_bta* m, int64_t nrhs);
 template <typename T>
-cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, cudaStream_t s);
+cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, int32_t* status,
+                        cudaStream_t s);
 
 // Whole-sweep triangular solve in one cluster launch (sgb_solve.cu).  `Li`
 // (n, b, b) holds the inverses of the diagonal sub-blocks of solve_sub() rows
 // of every L_ii at their places (their transposes with li_trans), `Lti` (a, a)
 // the same of the tip.  solve_chain_ok: whether the sizes fit it (otherwise
-// solve_chain returns cudaErrorNotSupported).
+// solve_chain returns cudaErrorNotSupported).  If a bounded wait gives up the
+// right-hand sides concerned become NaN and *status SGB_ERR_TIMEOUT.
 int solve_sub();
 template <typename T>
 bool solve_chain_ok(const sgb_bta* m, int64_t nrhs, cudaStream_t s);
 template <typename T>
 cudaError_t solve_chain(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, const T* Li, bool li_trans,
-                        const T* Lti, cudaStream_t s);
+                        const T* Lti, int32_t* status, cudaStream_t s);
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -440,6 +440,7 @@ struct SmallSolve {
     T* B;
     int64_t n, ldb, nrhs;
     int32_t b, a, trans;
+    int32_t* status;
 };
 
 template <typename T, int MB>
@@ -494,6 +495,7 @@ __global__ void __launch_bounds__(256) k_small_solve(const __grid_constant__ Sma
         S.tm[e / a][e % a] = A.Tp[e] * rd;
         if (e / a == e % a) S.trd[e % a] = rd;
     }
+    if (tid == 0 && blockIdx.x == 0) *A.status = 0;
     if (w >= 4) {
         fetch(0);
         park(0);
@@ -674,7 +676,8 @@ cudaError_t launch_solve(const SmallSolve<T>& A, cudaStream_t s) {
 }
 
 template <typename T>
-cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, cudaStream_t s) {
+cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, int32_t* status,
+                        cudaStream_t s) {
     SmallSolve<T> A;
     A.D = (const T*)m->diag;
     A.Lo = (const T*)m->lower;
@@ -687,6 +690,7 @@ cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool 
     A.b = (int32_t)m->b;
     A.a = (int32_t)m->a;
     A.trans = trans;
+    A.status = status;
     prof_before(s, SGB_KCLASS_GEMM);
     const cudaError_t e = m->b <= 16 ? launch_solve<T, 16>(A, s) : launch_solve<T, 32>(A, s);
     const double b = (double)m->b, a = (double)m->a;
@@ -696,7 +700,7 @@ cudaError_t small_solve(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool 
 
 #define SGB_INST(T)                                   \
     template bool small_solve_ok<T>(const sgb_bta*, int64_t);                                         \
-    template cudaError_t small_solve<T>(const sgb_bta*, T*, int64_t, int64_t, bool, cudaStream_t); \
+    template cudaError_t small_solve<T>(const sgb_bta*, T*, int64_t, int64_t, bool, int32_t*, cudaStream_t); \
     template bool small_factor_ok<T>(const sgb_bta*);  \
     template bool small_inverse_ok<T>(const sgb_bta*); \
     template cudaError_t small_inverse<T>(const sgb_bta*, int, int32_t*, cudaStream_t); \

@@ -77,7 +77,8 @@ struct SolveArgs {
     const T* Lti;  // (a, a): the same for the tip, never transposed
     T* B;
     int64_t n, ldb, nrhs;
-    long long spin;  // poll limit of every wait
+    int32_t* status;  // SGB_ERR_TIMEOUT if a wait gives up
+    long long spin;   // poll limit of every wait
     int32_t b, a;
     int32_t trans, li_trans;
     int32_t s, st;      // sub-block rows of a block and of the tip
@@ -618,6 +619,7 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
             volatile int never = 0;
             for (unsigned parity = 0; parity < 2; ++parity) bar_wait(bx + tid, parity, &never, 1 << 14);
         }
+        if (tid == 0) atomicExch(a.status, SGB_ERR_TIMEOUT);
         __syncthreads();
         const int64_t N = a.n * a.b + a.a;
         for (int64_t e = tid; e < N * nr; e += NT) a.B[(e / nr) * a.ldb + c0 + e % nr] = T(NAN);
@@ -749,7 +751,7 @@ bool solve_chain_ok(const sgb_bta* m, int64_t nrhs, cudaStream_t s) {
 
 template <typename T>
 cudaError_t solve_chain(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool trans, const T* Li, bool li_trans,
-                        const T* Lti, cudaStream_t s) {
+                        const T* Lti, int32_t* status, cudaStream_t s) {
     SolveArgs<T> a;
     Shape h;
     cudaError_t e = shape_of<T>(m, nrhs, s, a, h);
@@ -764,6 +766,7 @@ cudaError_t solve_chain(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool 
     a.ldb = ldb;
     a.trans = trans;
     a.li_trans = li_trans;
+    a.status = status;
     a.spin = spin_limit();
     a.warm = (double)a.n * a.b * (2.0 * a.b + a.a) * sizeof(T) > 48e6;
     cudaLaunchConfig_t cfg;
@@ -783,7 +786,7 @@ cudaError_t solve_chain(const sgb_bta* m, T* B, int64_t nrhs, int64_t ldb, bool 
 #define SGB_INST(T)                                                                                       \
     template bool solve_chain_ok<T>(const sgb_bta*, int64_t, cudaStream_t);                               \
     template cudaError_t solve_chain<T>(const sgb_bta*, T*, int64_t, int64_t, bool, const T*, bool, const T*, \
-                                        cudaStream_t);
+                                        int32_t*, cudaStream_t);
 SGB_INST(double)
 SGB_INST(float)
 

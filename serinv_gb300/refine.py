@@ -20,7 +20,7 @@ import ctypes
 import torch
 
 from . import _lib
-from .algs import _bta_struct, _finish, _prepare, _ptr, _stream, _workspace
+from .algs import _bta_struct, _check_status, _finish, _prepare, _ptr, _stream, _workspace
 
 
 def bta_matvec(A_diagonal_blocks, A_lower_diagonal_blocks, A_lower_arrow_blocks, A_arrow_tip_block, x,
@@ -97,4 +97,5 @@ def pobtas_refine(A_diagonal_blocks, A_lower_diagonal_blocks, A_lower_arrow_bloc
         rc = lib.sgb_pobtas_refine(ctypes.byref(mA), ctypes.byref(mL), _ptr(Bt), nrhs, max(nrhs, 1), int(iters),
                                    ws.data_ptr(), nbytes.value, _stream(device))
         _lib.raise_for(rc, "pobtas_refine")
-        _finish(w)
+        if _finish(w):
+            _check_status(ws, _lib.SGB_PREC_NATIVE, "pobtas_refine", always=True)
