@@ -337,8 +337,9 @@ int sgb_batch_plan_create(const sgb_bta* mats, void* const* rhs, const int64_t* 
                           sgb_batch_plan** plan);
 /* As sgb_batch_plan_create, with two schedule parameters for an autotuner:
  * panel_ctas, the CTA count of the captured column-block launches (0
- * selects 48; a count too small for the kernel's roles, < 18, makes those
- * blocks take the launch-based tile sweep), and options: SGB_BATCH_TC_KSPLIT
+ * selects 48, or 24 when the batch is more than six times the work of its
+ * longest matrix; a count too small for the kernel's roles, < 18, makes
+ * those blocks take the launch-based tile sweep), and options: SGB_BATCH_TC_KSPLIT
  * lets the captured tensor-core products split K over thread-block clusters
  * (off by default: the other streams fill the GPU).  The workspace size
  * depends on neither.  Best used with CUDA_DEVICE_MAX_CONNECTIONS >= 32 in

@@ -16,13 +16,20 @@
 
 #include "sgb_internal.cuh"
 
-// CTAs of a captured column-block launch unless the plan asks otherwise: three
-// launches side by side on 152 SMs.  Ten CTAs of a launch have other roles, so 24
-// left the trailing update of a block to 14.  ms a replay on 12 streams with 24,
-// 40, 48 and 64 CTAs: 12 matrices up to n=96 b=256, half of them FP32, mixed 34.9,
-// 29.7, 29.9, 30.5 and FP64 51.1, 38.8, 36.9, 37.4; 24 up to n=48 mixed 19.6, 18.6,
-// 19.2, 21.3; 4 up to n=40 mixed 14.1, 11.4, 11.2, 10.7.
-constexpr int kPlanPanelGrid = 48;
+// CTAs of a captured column-block launch unless the plan asks otherwise.  Ten of a
+// launch's CTAs have other roles, so 24 leave the trailing update of a block to 14;
+// with 48 three launches fill the 152 SMs, and the others' wait.  Where few
+// matrices make up most of the work their chain is what the replay waits for, and it
+// is shorter with 48; with many of a size the SMs are what is short.  ms a replay
+// with 24 and 48 CTAs, mixed and FP64 (every second matrix FP32), by the work of the
+// batch over that of its longest matrix: 1.3 (4 up to n=96 b=256) 33.5, 26.6 and
+// 52.5, 36.4; 2.7 (12 up to n=96 b=256) 34.5, 29.3 and 54.0, 39.8; 4.8 (24 up to
+// n=64 b=256) 25.6, 24.9 and 39.5, 34.6; 7.0 (24 up to n=48 b=256) 10.2, 12.4 and
+// 14.4, 14.2; 9.2 (48 up to n=48 b=256) 26.2, 29.1 and 41.6, 41.4; 11.5 (48 up to
+// n=32 b=128) 7.0, 8.4 and 6.9, 8.3; 29 (64 up to n=32 b=128) 14.3, 18.4 and 13.5,
+// 17.6.
+constexpr int kPlanPanelGrid = 48, kPlanPanelGridMany = 24;
+constexpr double kPlanMany = 6.0;
 
 struct sgb_batch_plan {
     int count = 0;
@@ -83,6 +90,15 @@ int validate(const sgb_bta* mats, void* const* rhs, const int64_t* nrhs, int cou
         it.ws = item_ws(it, ops);
     }
     return SGB_OK;
+}
+
+int panel_grid(const std::vector<Item>& items) {
+    double sum = 0.0, longest = 0.0;
+    for (const Item& it : items) {
+        sum += it.cost;
+        longest = std::max(longest, it.cost);
+    }
+    return sum > kPlanMany * longest ? kPlanPanelGridMany : kPlanPanelGrid;
 }
 
 // LPT assignment: biggest first onto the least loaded stream.
@@ -150,11 +166,11 @@ int sgb_batch_plan_create_ex(const sgb_bta* mats, void* const* rhs, const int64_
     if (!out || nstreams < 1 || nstreams > 256) return SGB_ERR_ARG;
     if (panel_ctas < 0 || panel_ctas > 1024) return SGB_ERR_ARG;
     if ((options & ~SGB_BATCH_TC_KSPLIT) != 0) return SGB_ERR_ARG;
-    const int pgrid = panel_ctas == 0 ? kPlanPanelGrid : panel_ctas;
     *out = nullptr;
     std::vector<Item> items;
     int rc = validate(mats, rhs, nrhs, count, ops, precisions, items);
     if (rc) return rc;
+    const int pgrid = panel_ctas == 0 ? panel_grid(items) : panel_ctas;
     const int ns = std::max(1, std::min(nstreams, count));
     const std::vector<int> where = assign(items, ns);
     const Layout L = layout(items, where, ns);
