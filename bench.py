@@ -578,7 +578,7 @@ def bench_batched(args):
             "dtype": "half f32, half " + ("f64 mixed" if args.batch_precision == "mixed" else "f64"),
             "data": "synthetic (NumPy generator, seed i for matrix i)",
             "config": {"workload": "batch of 256 uneven BTA matrices", "nstreams": ns,
-                       "panel_ctas": panel or 24, "tc_ksplit": split, "autotune_s": tune_s, "not_spd": bad,
+                       "panel_ctas": panel or "plan's own", "tc_ksplit": split, "autotune_s": tune_s, "not_spd": bad,
                        "hardware_queues": os.environ.get("CUDA_DEVICE_MAX_CONNECTIONS")},
             "max_rel_err_vs_single_fp64": {**worst, "vs": "single-matrix FP64 GPU path on the same inputs, "
                                                          "max over items of the relative Frobenius error of "

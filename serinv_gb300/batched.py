@@ -14,8 +14,8 @@ factor, then the selected inversion).
 schedules on scratch copies of the same shapes -- the worker-stream count,
 then the CTA count of the captured column-block launches, then whether the
 tensor-core products split K over clusters -- and caches the winner in a
-JSON file keyed by the batch signature, the device and the hardware-queue
-count (``CUDA_DEVICE_MAX_CONNECTIONS``), so the user's data is never
+JSON file keyed by the batch signature, the device, the hardware-queue
+count (``CUDA_DEVICE_MAX_CONNECTIONS``) and ``SCHEDULE``, so the user's data is never
 touched while tuning.
 """
 
@@ -33,7 +33,8 @@ from .algs import _bta_struct
 
 _OPS = {"pobtaf": 1, "pobtasi": 2, "pobtas": 4}
 CANDIDATES = (8, 16, 32, 64, 128)
-PANEL_CANDIDATES = (18, 26, 34, 64)  # beside the default, 48
+PANEL_CANDIDATES = (18, 24, 34, 48)  # beside the plan's own choice
+SCHEDULE = 2  # raised when a cached choice may no longer be the best: kernels or defaults have changed
 CACHE = os.environ.get("SGB_AUTOTUNE_CACHE",
                        os.path.join(os.path.expanduser("~"), ".cache", "serinv_gb300", "batch_autotune.json"))
 
@@ -45,7 +46,7 @@ def _signature(mats, rhs, ops, precisions) -> str:
         parts.append(f"{D.shape[0]}x{D.shape[1]}x{Ar.shape[1]}:{str(D.dtype)[6:]}:{nr}:{precisions[i]}")
     dev = torch.cuda.get_device_name(mats[0][0].device) if mats else ""
     conn = os.environ.get("CUDA_DEVICE_MAX_CONNECTIONS", "8")
-    key = ";".join(parts) + f"|ops={ops}|dev={dev}|conn={conn}"
+    key = ";".join(parts) + f"|ops={ops}|dev={dev}|conn={conn}|schedule={SCHEDULE}"
     return hashlib.sha1(key.encode()).hexdigest()
 
 
@@ -150,8 +151,8 @@ def autotune(mats, rhs=None, ops=("pobtaf", "pobtasi", "pobtas"), precisions=Non
              panel_candidates=PANEL_CANDIDATES, reps: int = 2):
     """Pick (worker-stream count, column-block CTA count, tensor-core K
     split) by timing warm replays on scratch copies of the batch: the stream
-    count first (the default CTA count, no K split), then the CTA count at that
-    stream count, then the K split.  Cached by signature."""
+    count first (the plan's own CTA count, no K split), then the CTA count at that
+    stream count (0: the plan's own), then the K split.  Cached by signature."""
     if precisions is None:
         precisions = ["fp64"] * len(mats)
     opcode = sum(_OPS[o] for o in ops)
@@ -175,9 +176,9 @@ def autotune(mats, rhs=None, ops=("pobtaf", "pobtasi", "pobtas"), precisions=Non
         if t < best_t:
             best_ns, best_t = ns, t
     best_panel = 0
-    for pc in panel_candidates:
-        if pc == 24:  # never the best: between 18 and the default, at which the stream search ran
-            continue
+    # (blocks of up to 64 have no column-block launches in a plan)
+    wide = any(m[0].shape[1] * (2 if m[0].is_complex() else 1) > 64 for m in mats)
+    for pc in panel_candidates if wide else ():
         t = _time_plan(mats, rhs, scratch, srhs, ops, precisions, best_ns, pc, reps)
         if t < best_t:
             best_panel, best_t = pc, t
