@@ -629,21 +629,36 @@ bool overlaps(const GemmProb<T>& p, const T* X, int64_t rows, int64_t cols, int6
     return off < p.N || off + cols > ld;
 }
 
-// 0: no operand overlaps its problem's output; 1: some do, and a tile of 32
-// columns holds their whole rows; 2: otherwise.
+// Whether row i of op(A) = A meets no row of the output but row i, in every
+// instance: then a CTA with whole rows of the output may write them in place.
+template <typename T>
+bool same_rows(const GemmProb<T>& p, const GemmTerm<T>& g) {
+    const int64_t bytes = (int64_t)((uintptr_t)g.A - (uintptr_t)p.Cout), off = bytes / (int64_t)sizeof(T);
+    if (g.transA || g.lda != p.ldc || bytes % (int64_t)sizeof(T) != 0 || (p.batch > 1 && g.strideA != p.strideC))
+        return false;
+    const int64_t rows = (p.M - 1) * p.ldc;  // from one instance to the next no less than the rows of one
+    if (p.batch > 1 && p.strideC < rows + (off > 0 ? off : 0) + (g.K > p.N ? g.K : p.N)) return false;
+    return off >= 0 ? off + g.K <= p.ldc : p.N - off <= p.ldc;
+}
+
+// 0: no operand overlaps its problem's output; 1: rows of A do, each its own row
+// (same_rows), and a tile of 32 columns holds whole rows of the output; 2: some
+// other way, for which a launch of more than one tile has no order that helps:
+// it gets the 32 x 32 tiles, of which one holds an output of up to 32 x 32.
 template <typename T>
 int in_place(const GemmProb<T>* probs, int np) {
     int worst = 0;
     for (int i = 0; i < np; ++i) {
         const GemmProb<T>& p = probs[i];
         if (p.M <= 0 || p.N <= 0 || p.batch <= 0) continue;
-        bool over = p.Cin != nullptr && p.transCin;
+        if (p.Cin != nullptr && p.transCin && overlaps<T>(p, p.Cin, p.N, p.M, p.ldcin, p.strideCin)) return 2;
         for (int t = 0; t < p.nterms; ++t) {
             const GemmTerm<T>& g = p.term[t];
-            over = over || overlaps<T>(p, g.A, g.transA ? g.K : p.M, g.transA ? p.M : g.K, g.lda, g.strideA) ||
-                   overlaps<T>(p, g.B, g.transB ? p.N : g.K, g.transB ? g.K : p.N, g.ldb, g.strideB);
+            if (overlaps<T>(p, g.B, g.transB ? p.N : g.K, g.transB ? g.K : p.N, g.ldb, g.strideB)) return 2;
+            if (!overlaps<T>(p, g.A, g.transA ? g.K : p.M, g.transA ? p.M : g.K, g.lda, g.strideA)) continue;
+            if (p.N > 32 || !same_rows<T>(p, g)) return 2;
+            worst = 1;
         }
-        if (over) worst = p.N <= 32 && worst < 2 ? 1 : 2;
     }
     return worst;
 }
