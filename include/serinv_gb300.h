@@ -119,6 +119,13 @@ int sgb_last_cuda_error(void);
 int sgb_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes);
 int sgb_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes);
 int sgb_pobtas_workspace_size(const sgb_bta* m, int64_t nrhs, int precision, size_t* bytes);
+/*
+ * The least workspace a call runs in: op SGB_OP_POBTAF or SGB_OP_POBTASI, ring < 0
+ * for the plain and host forms, otherwise the streamed form's ring.  Below the
+ * sizes above by the slice buffers of SGB_PREC_NATIVE; without them all products
+ * are FP64 sums.
+ */
+int sgb_least_workspace_size(const sgb_bta* m, int op, int precision, int64_t ring, size_t* bytes);
 
 /*
  * In-place block Cholesky A = L L^T.
@@ -264,11 +271,11 @@ int sgb_pobtas_refine(const sgb_bta* A, const sgb_bta* L, void* rhs, int64_t nrh
  * loops that forbid allocator calls, and foreign-language hosts that hold
  * device pointers but no allocator.  This entry point has no counterpart in
  * the reference; it computes exactly what sgb_pobtaf with precision
- * SGB_PREC_NATIVE computes.
+ * SGB_PREC_NATIVE and the least workspace computes (all products FP64 sums).
  *
  * Its scratch is a static device array of sgb_pobtaf_noalloc_scratch_bytes()
  * bytes (128 KiB) that every GPU loading the library keeps until the process
- * exits.  Requests whose workspace (sgb_pobtaf_workspace_size) exceeds it
+ * exits.  Requests whose least workspace (sgb_least_workspace_size) exceeds it
  * return SGB_ERR_WORKSPACE.  The first call on a device looks up the array's
  * device address (cudaGetSymbolAddress) with that device current; make that
  * first call before any stream capture.  All calls share the array: calls

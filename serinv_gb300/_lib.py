@@ -30,6 +30,8 @@ SGB_C64 = 2
 SGB_C128 = 3
 
 SGB_BATCH_TC_KSPLIT = 1
+SGB_OP_POBTAF = 1
+SGB_OP_POBTASI = 2
 
 SGB_PREC_NATIVE = 0
 SGB_PREC_MIXED = 1
@@ -87,6 +89,8 @@ _SIGNATURES = {
                                   ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p]),
     "sgb_pobtasi": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_int, ctypes.c_int, ctypes.c_void_p,
                                    ctypes.c_size_t, ctypes.c_void_p]),
+    "sgb_least_workspace_size": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_int, ctypes.c_int,
+                                                ctypes.c_int64, ctypes.POINTER(ctypes.c_size_t)]),
     "sgb_pobtasi_has_waits": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_int]),
     "sgb_pobtas": (ctypes.c_int, [ctypes.POINTER(SgbBta), ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64,
                                   ctypes.c_char, ctypes.c_int, ctypes.c_int, ctypes.c_void_p,

@@ -172,6 +172,20 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
 
 
+def _sweep_workspace(m, op: int, precision: int, nbytes: int, device, ring: int = -1):
+    """A workspace of nbytes, or where that does not fit into the device's memory
+    the least one the call runs in; and its size."""
+    try:
+        return _workspace(nbytes, device), nbytes
+    except torch.OutOfMemoryError:
+        least = ctypes.c_size_t(0)
+        _lib.raise_for(_lib.load().sgb_least_workspace_size(ctypes.byref(m), op, precision, int(ring),
+                                                            ctypes.byref(least)), "workspace")
+        if least.value >= nbytes:
+            raise
+    return _workspace(least.value, device), least.value
+
+
 def _check_status(ws: torch.Tensor, precision: int, what: str, always: bool = False) -> None:
     """The workspace's first int32 is the device status word (bounded waits)."""
     if not always and (precision & 0xFF) != _lib.SGB_PREC_MIXED:
@@ -269,8 +283,9 @@ def _stream_call(entry, size_query, host, what, precision, flag, ring, with_info
     with torch.cuda.device(device):
         nbytes = ctypes.c_size_t(0)
         _lib.raise_for(size_query(ctypes.byref(mh), precision, int(ring), ctypes.byref(nbytes)), what)
-        ws = _workspace(nbytes.value, device)
-        args = [ctypes.byref(mh), int(flag), precision, int(ring), ws.data_ptr(), nbytes.value]
+        op = _lib.SGB_OP_POBTAF if with_info else _lib.SGB_OP_POBTASI
+        ws, size = _sweep_workspace(mh, op, precision, nbytes.value, device, max(int(ring), 0))
+        args = [ctypes.byref(mh), int(flag), precision, int(ring), ws.data_ptr(), size]
         info = torch.zeros(1, dtype=torch.int32, device=device) if with_info else None
         if with_info:
             args.append(info.data_ptr())
@@ -292,8 +307,9 @@ def _host_call(entry, size_query, host, what, precision, flag, with_info):
     with torch.cuda.device(device):
         nbytes = ctypes.c_size_t(0)
         _lib.raise_for(size_query(ctypes.byref(md), precision, ctypes.byref(nbytes)), what)
-        ws = _workspace(nbytes.value, device)
-        args = [ctypes.byref(mh), ctypes.byref(md), int(flag), precision, ws.data_ptr(), nbytes.value]
+        op = _lib.SGB_OP_POBTAF if with_info else _lib.SGB_OP_POBTASI
+        ws, size = _sweep_workspace(md, op, precision, nbytes.value, device)
+        args = [ctypes.byref(mh), ctypes.byref(md), int(flag), precision, ws.data_ptr(), size]
         info = torch.zeros(1, dtype=torch.int32, device=device) if with_info else None
         if with_info:
             args.append(info.data_ptr())
@@ -367,11 +383,11 @@ def pobtaf(A_diagonal_blocks, A_lower_diagonal_blocks, A_lower_arrow_blocks, A_a
         nbytes = ctypes.c_size_t(0)
         _lib.raise_for(lib.sgb_pobtaf_workspace_size(ctypes.byref(m), precision, ctypes.byref(nbytes)),
                        "pobtaf")
-        ws = _workspace(nbytes.value, device)
+        ws, size = _sweep_workspace(m, _lib.SGB_OP_POBTAF, precision, nbytes.value, device)
         # the second word of the status slot, set by the call itself: one read
         # tells both, and no buffer is made and cleared for it
         rc = lib.sgb_pobtaf(ctypes.byref(m), int(factorize_last_block), precision, ws.data_ptr(),
-                            nbytes.value, ws.data_ptr() + 4, _stream(device))
+                            size, ws.data_ptr() + 4, _stream(device))
         _lib.raise_for(rc, "pobtaf")
         _finish(w)
         if check:
@@ -432,8 +448,8 @@ def pobtasi(L_diagonal_blocks, L_lower_diagonal_blocks, L_lower_arrow_blocks, L_
         nbytes = ctypes.c_size_t(0)
         _lib.raise_for(lib.sgb_pobtasi_workspace_size(ctypes.byref(m), precision, ctypes.byref(nbytes)),
                        "pobtasi")
-        ws = _workspace(nbytes.value, device)
-        rc = lib.sgb_pobtasi(ctypes.byref(m), int(invert_last_block), precision, ws.data_ptr(), nbytes.value,
+        ws, size = _sweep_workspace(m, _lib.SGB_OP_POBTASI, precision, nbytes.value, device)
+        rc = lib.sgb_pobtasi(ctypes.byref(m), int(invert_last_block), precision, ws.data_ptr(), size,
                              _stream(device))
         _lib.raise_for(rc, "pobtasi")
         waits = lib.sgb_pobtasi_has_waits(ctypes.byref(m), precision) and bool(kwargs.get("check_spd", True)) \

@@ -318,7 +318,7 @@ struct PobtasiWs {
             const int64_t tb = chunk < kSiTcBatch ? chunk : kSiTcBatch;
             size_t need[5];
             need[0] = tc_prob_bytes(S, b, b, kba, 1) + tc_prob_bytes(S, a, b, kba, 1);  // back-sweep step
-            need[1] = 2 * tc_prob_bytes(S, b, b, b, tb) + tc_prob_bytes(S, a, b, b, tb);  // G, P, H
+            need[1] = (S > 7 ? 1 : 2) * tc_prob_bytes(S, b, b, b, tb) + tc_prob_bytes(S, a, b, b, tb);  // G, H, (S <= 7) P
             need[2] = trtri_tc_bytes(S, b, chunk);
             need[3] = trtri_tc_bytes(S, a, 1);
             need[4] = tc_prob_bytes(S, a, a, a, 1);  // tip
@@ -1647,13 +1647,6 @@ bool item_keeps_inverses(const sgb_bta* m, int precision, int ops) {
 
 }  // namespace
 
-int pobtaf_least_workspace(const sgb_bta* m, size_t* bytes) {
-    if (cx_dtype(m)) return sgb_pobtaf_workspace_size(m, SGB_PREC_NATIVE, bytes);
-    const int rc = check_bta(m);
-    if (rc == SGB_OK) *bytes = taf_bytes(m, 0, 0);
-    return rc;
-}
-
 size_t plan_item_ws(const sgb_bta* m, int ops, int precision, int64_t nrhs) {
     size_t need = 0, x = 0;
     if (ops & SGB_OP_POBTAF) {
@@ -1928,6 +1921,30 @@ int sgb_pobtaf(const sgb_bta* m, int factorize_last_block, int precision, void* 
     return pobtaf_run<float>(m, factorize_last_block, S, Si, workspace, info, s);
 }
 
+int sgb_least_workspace_size(const sgb_bta* m, int op, int precision, int64_t ring, size_t* bytes) {
+    if (op != SGB_OP_POBTAF && op != SGB_OP_POBTASI) return SGB_ERR_ARG;
+    const bool inverse = op == SGB_OP_POBTASI;
+    if (cx_dtype(m)) {
+        if (ring >= 0) return SGB_ERR_UNSUPPORTED;
+        return inverse ? cx_pobtasi_workspace_size(m, precision, bytes, false, true)
+                       : cx_pobtaf_workspace_size(m, precision, bytes, false, true);
+    }
+    const int rc = check_bta(m);
+    if (rc) return rc;
+    const int S = parse_precision(precision, m->dtype);
+    if (S < 0) return -S;
+    if (!bytes) return SGB_ERR_ARG;
+    if (ring >= 0) {
+        int slices = 0;
+        int64_t R = 0;
+        size_t sweep = 0;
+        return stream_sizes(m, precision, ring, inverse, 0, &slices, &R, &sweep, bytes);
+    }
+    const int Si = parse_inv_slices(precision, S);
+    *bytes = inverse ? tasi_bytes(m, S, Si) : taf_bytes(m, S, Si);
+    return SGB_OK;
+}
+
 int sgb_pobtasi_has_waits(const sgb_bta* m, int precision) {
     if (m == nullptr) return 0;
     sgb_bta r = *m;
@@ -1998,9 +2015,7 @@ int sgb_pobtaf_permuted(const sgb_bta* m, void* buffer, int precision, void* wor
     const int Si = parse_inv_slices(precision, S);
     if (m->n < 2) return SGB_ERR_SHAPE;
     if (buffer == nullptr) return SGB_ERR_ARG;
-    size_t need = 0;
-    sgb_pobtaf_permuted_workspace_size(m, precision, &need);
-    if ((rc = check_ws(workspace, workspace_bytes, need))) return rc;
+    if ((rc = check_ws(workspace, workspace_bytes, taf_bytes(m, S, Si)))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     if (info) SGB_TRY(cudaMemsetAsync(info, 0, sizeof(int32_t), s));
     SGB_TRY(cudaMemsetAsync(workspace, 0, kStatusBytes, s));

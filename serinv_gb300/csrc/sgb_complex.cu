@@ -266,20 +266,22 @@ bool cx_dtype(const sgb_bta* m) { return m != nullptr && is_complex(m->dtype); }
 
 // ---- workspace queries -------------------------------------------------
 
-int cx_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted) {
+int cx_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted, bool least) {
     sgb_bta r = real_desc(m);
     size_t rb = 0;
-    int rc = sgb_pobtaf_workspace_size(&r, precision, &rb);
+    int rc = least ? sgb_least_workspace_size(&r, SGB_OP_POBTAF, precision, -1, &rb)
+                   : sgb_pobtaf_workspace_size(&r, precision, &rb);
     if (rc) return rc;
     if (!bytes) return SGB_ERR_ARG;
     *bytes = CxLayout(r, rb, permuted, 0).total;
     return SGB_OK;
 }
 
-int cx_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted) {
+int cx_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted, bool least) {
     sgb_bta r = real_desc(m);
     size_t rb = 0;
     int rc = permuted ? sgb_pobtasi_permuted_workspace_size(&r, precision, &rb)
+             : least  ? sgb_least_workspace_size(&r, SGB_OP_POBTASI, precision, -1, &rb)
                       : sgb_pobtasi_workspace_size(&r, precision, &rb);
     if (rc) return rc;
     if (!bytes) return SGB_ERR_ARG;
@@ -306,6 +308,9 @@ int cx_pobtaf_t(const sgb_bta* m, int flb, int precision, void* ws, size_t ws_by
     size_t rb = 0;
     int rc = sgb_pobtaf_workspace_size(&r, precision, &rb);
     if (rc) return rc;
+    // a workspace without room for the slices of the native form will do
+    if (ws_bytes < CxLayout(r, rb, buffer != nullptr, 0).total)
+        sgb_least_workspace_size(&r, SGB_OP_POBTAF, precision, -1, &rb);
     CxLayout L(r, rb, buffer != nullptr, 0);
     if ((rc = check_ws(ws, ws_bytes, L.total))) return rc;
     if ((rc = embed_all<T>(m, r, L, ws, 1, buffer, s))) return rc;
@@ -331,6 +336,8 @@ int cx_pobtasi_t(const sgb_bta* m, int ilb, int precision, void* ws, size_t ws_b
     int rc = buffer ? sgb_pobtasi_permuted_workspace_size(&r, precision, &rb)
                     : sgb_pobtasi_workspace_size(&r, precision, &rb);
     if (rc) return rc;
+    if (!buffer && ws_bytes < CxLayout(r, rb, false, 0).total)
+        sgb_least_workspace_size(&r, SGB_OP_POBTASI, precision, -1, &rb);
     CxLayout L(r, rb, buffer != nullptr, 0);
     if ((rc = check_ws(ws, ws_bytes, L.total))) return rc;
     if ((rc = embed_all<T>(m, r, L, ws, 0, buffer, s))) return rc;

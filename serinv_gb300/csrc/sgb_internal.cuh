@@ -237,9 +237,6 @@ cudaError_t bta_symv(const sgb_bta* A, const T* x, int64_t ldx, T* y, int64_t ld
 template <typename T>
 cudaError_t axpy2d(T* x, int64_t ldx, const T* y, int64_t ldy, int64_t rows, int64_t cols, cudaStream_t s);
 
-// Workspace a native pobtaf runs in without the exact slice products.
-int pobtaf_least_workspace(const sgb_bta* m, size_t* bytes);
-
 // One matrix of a batch plan (sgb_api.cu): its workspace size and the ops.
 size_t plan_item_ws(const sgb_bta* m, int ops, int precision, int64_t nrhs);
 int plan_item(const sgb_bta* m, int ops, int precision, void* rhs, int64_t nrhs, void* ws, size_t wsb,
@@ -251,8 +248,8 @@ int record_cuda_error(cudaError_t e);
 // Complex dtypes through the real embedding (sgb_complex.cu).  buffer !=
 // nullptr selects the permuted form.
 bool cx_dtype(const sgb_bta* m);
-int cx_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted);
-int cx_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted);
+int cx_pobtaf_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted, bool least = false);
+int cx_pobtasi_workspace_size(const sgb_bta* m, int precision, size_t* bytes, bool permuted, bool least = false);
 int cx_pobtas_workspace_size(const sgb_bta* m, int64_t nrhs, int precision, size_t* bytes, bool permuted);
 int cx_pobtaf(const sgb_bta* m, int flb, int precision, void* ws, size_t ws_bytes, int32_t* info, cudaStream_t s,
               void* buffer);

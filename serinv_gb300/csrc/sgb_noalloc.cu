@@ -81,7 +81,7 @@ size_t sgb_pobtaf_noalloc_scratch_bytes(void) { return kStaticScratchBytes; }
 
 int sgb_pobtaf_noalloc(const sgb_bta* m, int factorize_last_block, int32_t* info, void* stream) {
     size_t need = 0;
-    int rc = sgb::pobtaf_least_workspace(m, &need);
+    int rc = sgb_least_workspace_size(m, SGB_OP_POBTAF, SGB_PREC_NATIVE, -1, &need);
     if (rc != SGB_OK) return rc;
     if (need > kStaticScratchBytes) return SGB_ERR_WORKSPACE;
     void* scratch = nullptr;
