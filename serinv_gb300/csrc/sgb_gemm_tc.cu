@@ -13,7 +13,10 @@
 // 2^(-7l) whose magnitude stays below 2^24 of those units: per k a level-l
 // term is at most 2^14 + (l-1) 2^12 units, so levels 0..4 are exact for
 // K <= kTcMaxK = 576.  Each level up to 4 has its own TMEM accumulator; for
-// S = 7 the last accumulator also takes levels 5 and 6 (weight <= 2^-35).
+// S = 7 the last accumulator also takes levels 5 and 6 (weight <= 2^-35).  For
+// S = 9 level 5 has its own, exact for K <= 512; past that a sum of digits all at
+// their bounds could round by a unit, 2^-47 2^(EA + EB), where the element itself is
+// some 2^9 2^(EA + EB).
 // The truncation error of S digits is 2^-(7S+1) of the row maximum.  The
 // epilogue adds the accumulators exactly as an FP32 pair (two-sum), widens
 // the pair with integer bit operations, adds it in FP64 (one FP64 add),
@@ -980,8 +983,9 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
     };
     // Exact form: the level sums as integers in units of 2^-45 -- level 0, up to
     // 2^24 2^45, apart from the others, whose sum stays below 2^62 -- so that
-    // adding levels and the CTAs of a K split rounds nothing (levels 6 to 8 share
-    // an accumulator, rounded to a unit); one FMA at the end rounds to FP64.
+    // adding the levels as they stand in TMEM and the CTAs of a K split rounds
+    // nothing (levels 6 to 8 share an accumulator, rounded to a unit); one FMA at
+    // the end rounds to FP64.
     auto fold = [&](const float (&vv)[NACC], int& i0, long long& t) {
         i0 = __float2int_rn(vv[0]);
         t = 0;
@@ -1296,7 +1300,8 @@ __global__ void __launch_bounds__(TC_THREADS2, 1) k_gemm_tc(const __grid_constan
             }
         }
     }
-    // a wait gave up: this CTA's part of the tile is marked
+    // a wait gave up: the tile is marked (a peer that went on may still write its rows;
+    // the status word tells)
     if (!all_ok)
         for (int e = tid; e < TC_BM * BN; e += TC_THREADS2) store(e / BN, e % BN, __longlong_as_double(0x7ff8000000000000ll), 0.0);
     if (!all_ok && tid == 0) {

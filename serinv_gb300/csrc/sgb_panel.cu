@@ -186,19 +186,16 @@ __device__ __forceinline__ T* row_ptr(const PanelArgs<T>& a, int64_t c1, int64_t
 // columns of M (transposed in mt) and d^{-1/2} (rv) are consumed as the
 // factorizer publishes them: column k once *colcount >= col_base + k + 1
 // (bounded wait; `sleep` backs off between polls), all available columns
-// loaded at once.  With stage_row the result also goes to that staging row
-// (hand-off by value).  With unit >= 0
-// the row is the unit vector e_unit instead of the stored values (a row of
-// the identity, whose solve is a row of L^{-T}); with preset the row starts
-// from y0 (lane = column) instead.  With kApart the products are summed by
-// themselves and taken from the row at once (one more instruction a column):
-// in sequence each rounds at the row's size.  Returns false on a timeout or an
-// error raised elsewhere.
+// loaded at once.  With unit >= 0 the row is the unit vector e_unit instead of
+// the stored values (a row of the identity, whose solve is a row of L^{-T}); with
+// preset the row starts from y0 (lane = column) instead.  With kApart the products
+// are summed by themselves and taken from the row at once (one more instruction a
+// column): in sequence each rounds at the row's size.  Returns false on a timeout
+// or an error raised elsewhere.
 template <typename T, bool kApart>
 __device__ __forceinline__ bool trsm_row_pipe(T* rp, int w, const T* mt, const T* rv, const unsigned* colcount,
                                               unsigned col_base, int32_t* status, bool sleep, long long spin,
-                                              int unit = -1, T* stage_row = nullptr, bool preset = false,
-                                              T y0 = T(0)) {
+                                              int unit = -1, bool preset = false, T y0 = T(0)) {
     const int tx = threadIdx.x & 31;
     T y = tx < w ? (unit >= 0 ? T(tx == unit ? 1 : 0) : preset ? y0 : ldcg(rp + tx)) : T(0);
     const T start = y;
@@ -247,11 +244,7 @@ __device__ __forceinline__ bool trsm_row_pipe(T* rp, int w, const T* mt, const T
             k += nb;
         }
     }
-    if (tx < w) {
-        const T x = y * r;
-        rp[tx] = x;
-        if (stage_row != nullptr) stage_put(stage_row + tx, x);
-    }
+    if (tx < w) rp[tx] = y * r;
     return true;
 }
 
@@ -634,8 +627,8 @@ __global__ void __launch_bounds__(NT, 1) k_factor_panel(const __grid_constant__ 
                 for (int k = 0; k < kTile; ++k) s = fma(-__shfl_sync(0xffffffffu, av, k), tr[tx][k], s);
                 y0 = kApart ? y0 + s : s;
             }
-            return trsm_row_pipe<T, kApart>(rp, w, Mp, rp3, CC, (unsigned)(p * kTile), a.status, true, a.spin, unit, nullptr,
-                                    prev && unit < 0, y0);
+            return trsm_row_pipe<T, kApart>(rp, w, Mp, rp3, CC, (unsigned)(p * kTile), a.status, true, a.spin, unit,
+                                            prev && unit < 0, y0);
         };
         if (ty < 4) {
             if (prev) {
