@@ -88,9 +88,9 @@ int parse_inv_slices(int precision, int S) {
 // Below the lines the slicing and the longer epilogue cost more than the FP64
 // pipe's 16 x 16 tiles.  ms, exact slices and FP64 pipe: factorization n=64 b=160
 // a=0 5.77 / 5.38, b=192 a=16 6.68 / 6.47, a=64 6.80 / 7.00, b=208 7.17 / 7.10, b=224
-// 7.50 / 7.71, b=256 a=32 8.43 / 9.59, b=512 a=64 20.7 / 31.3; selected inverse n=64
-// b=176 3.75 / 3.70, b=192 a=16 4.07 / 4.25, a=64 4.17 / 5.15, b=224 4.46 / 5.59,
-// b=512 a=64 13.2 / 53.4.  With fewer blocks the inversions ahead of the back-sweep
+// 7.50 / 7.71, b=256 a=32 8.43 / 9.59, b=512 a=64 20.6 / 31.3; selected inverse n=64
+// b=176 3.75 / 3.70, b=192 a=0 3.83 / 3.99, a=64 4.23 / 5.15, b=224 4.44 / 5.59,
+// b=512 a=64 13.0 / 53.3.  With fewer blocks the inversions ahead of the back-sweep
 // weigh more: n=24 b=208 1.63 / 1.58, b=224 1.64 / 2.00, n=6 b=208 0.49 / 0.42, b=224
 // 0.50 / 0.52.
 constexpr int64_t kExactMin = 224, kExactMinInv = 192;  // the latter from 32 blocks on
@@ -953,7 +953,7 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
     cx.status = (int32_t*)(base + W.status);
     Ctx cxi = cx;  // the inversions and the products with L_ii^{-1}
     cxi.slices = Si ? Si : S;
-    Ctx cxt = cxi;  // without the exact slices: the tip, for which they do not pay, and P
+    Ctx cxt = cxi;  // without the exact slices: the tip, for which they do not pay, P and X_T H
     if (S > 7) cxt.slices = 0;
     T* Linv = (T*)(base + W.linv);
     T* Ltinv = (T*)(base + W.linv_tip);
@@ -1024,6 +1024,22 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 // matrix and would nearly all be summed on the FP64 pipe one by one
                 SGB_TRY(run_gemm<T>(cxi, pr, np, s));
                 np = 0;
+                if (a) {
+                    // -X_T H_j into Ar_j, which is dead: with the tip's diagonal as large as a
+                    // long chain makes it, a sum with X_{A,j+1} G_j in one product would lie far
+                    // below the largest entries of its row and column
+                    GemmProb<T> p = prob<T>();
+                    p.M = (int32_t)a;
+                    p.N = (int32_t)b;
+                    p.batch = (int32_t)jn;
+                    set_term<T>(p, 0, Tp, a, 0, GHj + bb, b, 0, a);
+                    p.term[0].strideB = ghs;
+                    p.alpha = T(-1);
+                    p.Cout = B.ar(j0);
+                    p.ldc = b;
+                    p.strideC = ab;
+                    pr[np++] = p;
+                }
             }
             {  // P_j = L_jj^{-T} L_jj^{-1} into D_j
                 GemmProb<T> p = prob<T>();
@@ -1061,7 +1077,7 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                 p.ldc = b;
                 pr[np++] = p;
             }
-            if (a) {  // X_{A,i} = -(X_{A,i+1} G_i + X_T H_i)  (:157-162, :128-130)
+            if (a && (has_next || S <= 7)) {  // X_{A,i} = -(X_{A,i+1} G_i + X_T H_i)  (:157-162, :128-130)
                 GemmProb<T> p = prob<T>();
                 p.M = (int32_t)a;
                 p.N = (int32_t)b;
@@ -1070,15 +1086,20 @@ int pobtasi_run(const sgb_bta* m, int invert_last_block, int S, int Si, void* ws
                     set_term<T>(p, t, B.ar(i + 1), b, 0, G, b, 0, b);
                     balance<T>(p, t++, B.d(i + 1), b);
                 }
-                set_term<T>(p, t, Tp, a, 0, H, b, 0, a);
-                balance<T>(p, t, Tp, a);
+                if (S <= 7) {
+                    set_term<T>(p, t, Tp, a, 0, H, b, 0, a);
+                } else {  // Ar_i holds -X_T H_i
+                    p.beta = T(1);
+                    p.Cin = B.ar(i);
+                    p.ldcin = b;
+                }
                 p.alpha = T(-1);
                 p.Cout = B.ar(i);
                 p.ldc = b;
                 pr[np++] = p;
             }
-            if (np > 0) {  // (a == 0 and no next block: X_ii = P_i)
-                SGB_TRY(run_gemm<T>(cx, pr, np, s));
+            if (np > 0) SGB_TRY(run_gemm<T>(cx, pr, np, s));
+            if (has_next || a) {  // (otherwise X_ii = P_i)
                 // X_ii = P_i - X_{i+1,i}^T G_i - X_{A,i}^T H_i  (:164-169, :133-137)
                 GemmProb<T> p = prob<T>();
                 p.M = p.N = (int32_t)b;

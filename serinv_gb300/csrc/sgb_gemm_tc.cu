@@ -45,11 +45,12 @@
 // with such matrices one element in 500 is below the line, with a decaying inverse
 // nearly all.  A warp sums single elements, 32 k at a time.  A CTA where these are
 // a quarter of the elements of most threads sums its whole part of the tile as FP64
-// tiles; and after a product in which most CTAs did, the slicing launches of the call's other products
-// form these so, spread over all SMs, instead of slicing.  ms, n=32, factorization
-// and selected inverse of matrices of decaying blocks, so and with the FP64 pipe's
-// own kernels: b=192 3.9, 3.2 and 3.2, 2.0; b=320 7.0, 8.9 and 6.6, 6.8; b=512 19.6,
-// 31.9 and 15.6, 26.3 (with single elements only 40, 156).
+// tiles; and after a product in which more than an eighth of the CTAs did (which
+// takes them as long as the pipe takes for the whole product), the slicing launches
+// of the call's other products form these so, spread over all SMs, instead of
+// slicing.  ms, n=32, factorization and selected inverse of matrices of decaying
+// blocks, so and with the FP64 pipe's own kernels: b=224 4.4, 4.1 and 3.9, 2.8; b=320 7.0, 8.3 and 6.7, 6.8; b=512 19.5,
+// 31.6 and 15.6, 26.4 (with single elements only 40, 156).
 //
 // This is the published Ozaki error-free splitting idea (Ozaki, Ogita,
 // Oishi, Rump) specialised to fixed-point digits and level-grouped exact
@@ -142,6 +143,7 @@ struct SplitJob {
 constexpr int kExpBias = 8192;  // keeps a scaled exponent positive
 constexpr int kExpOdd = -1;
 constexpr float kPipeBelow = 0x1p-5f;  // S = 9: elements below this share of 2^(EA + EB) go to the FP64 pipe
+constexpr int kPipeCtas = 152;  // CTAs of a slicing launch that form a product on the FP64 pipe: the SMs
 constexpr int kSplitRows = 8;
 constexpr int kSplitThreads = 512;  // two CTAs per SM, eight warps per scheduler: latency bound
 constexpr int kSplitLd = kTcMaxK + 1;  // odd stride: conflict-free row and column access
@@ -220,7 +222,7 @@ struct PipeMode {
     }
     __device__ __forceinline__ bool decide() const {
         const int32_t n = ((const volatile int32_t*)words)[SW_PARTS + ((number - 1) & 1)];
-        const bool pipe = noted() | (2 * n > before);
+        const bool pipe = noted() | (8 * n > before);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             words[SW_PARTS + (number & 1)] = 0;
             if (pipe && words[SW_PIPE] == 0) words[SW_PIPE] = number;
@@ -397,8 +399,11 @@ __global__ void __launch_bounds__(kSplitThreads, S > 7 ? 1 : 2)
     __shared__ short sk[kScaled ? kTcMaxK : 1];  // power of two of each k
     pdl_enter();
     if constexpr (kScaled) {
-        if (L.mode.decide()) {  // tiles of all problems, dealt to the CTAs in turn
-            const int ctas = (int)gridDim.x;
+        if (L.mode.decide()) {
+            // tiles of all problems, dealt in turn to as many CTAs as run at once (one an
+            // SM: dealt to all 208 of a launch they took 459 us for 313)
+            const int ctas = (int)gridDim.x < kPipeCtas ? (int)gridDim.x : kPipeCtas;
+            if ((int)blockIdx.x >= ctas) return;
             for (int q = 0, done = 0; q < W.np; ++q)
                 for (int i = 0; i < W.p[q].batch; ++i)
                     done += pipe_tiles<kSplitThreads / 256>(W.p[q], i, 0, W.p[q].M, 0, W.p[q].N,
@@ -1624,8 +1629,7 @@ cudaError_t gemm_tc(GemmProb<double>* probs, int np, int S, void* ws, size_t ws_
                 memcpy(W.p, TL.p, sizeof(W.p));
                 W.np = TL.np;
                 SL.strips = (int32_t)split_ctas;
-                e = launch_split<kExactSlices>(SL, shared_gpu || split_ctas > kTcSmCount ? (int)split_ctas : (int)kTcSmCount,
-                                               s, W);
+                e = launch_split<kExactSlices>(SL, shared_gpu || split_ctas > kPipeCtas ? (int)split_ctas : kPipeCtas, s, W);
             }
         }
         prof_after(SGB_KCLASS_SPLIT, s, 0.0);
