@@ -302,12 +302,12 @@ def replica_throughput(step_flops: float, world: int, per_step_s: float) -> floa
 
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from one ncu
-# capture of the same kernel at the same block sizes (the per-launch traffic
+# capture of the kernel in use at the same block sizes (the per-launch traffic
 # of one block step does not depend on n): key (kernel class, precision, b, a).
 # Source: profiles/launches_mixed_fp64_bench_n64_b512_a64.md (column-block
-# kernel DRAM traffic, launches 70-72).
+# kernel DRAM traffic, mean of launches 70-72).
 TRAFFIC_PER_LAUNCH = {
-    ("panel", "mixed", 512, 64): 1.24e6 + 0.6e3,
+    ("panel", "mixed", 512, 64): 1.25e6 + 0.9e3,
 }
 
 
