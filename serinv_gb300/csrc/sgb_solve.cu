@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
         const int o0 = 2 * w + half;  // this half warp's first own row
         constexpr int LC = 16 / NR;   // lanes that hold the same sum
         const int c = h / LC;
-        T la[KH], l1[KH];
+        T la[KH], l1[KH], ld;
         int f, cnt;
         // the CTAs this lane sends a sum to: base of their shared memory
         constexpr int NG = kMaxCluster / LC;
@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
             own_of(K.rows(sb), lg, rank, ff, cc);
             fetch_half<T>(la, M + (row_major ? (int64_t)(ff + o) * K.m : (int64_t)(ff + o)), row_major ? 1 : K.m, o < cc,
                           K.rows(sb));
+            ld = o < cc ? ld_now(M + (int64_t)(ff + o) * (K.m + 1)) : T(0);
         };
         fetch_inv(cur, tr ? cur.nsub - 1 : 0, o0);
         for (int64_t j = jfirst;; j += dj) {
@@ -410,8 +411,14 @@ __global__ void __launch_bounds__(NT, 1) k_solve(const __grid_constant__ SolveAr
                     if (o != o0) fetch_inv(cur, q, o);
                     T v[NR];
                     const T* xs = step > 0 ? xbuf + (p ^ 1) * kBuf : xbuf;
-                    mults_half<T, NR>(v, la, xs, K, tr ? f + o : 0, tr ? K : f + o + 1);
+                    // the diagonal's term by itself and last: in the lanes' sums four more of
+                    // them would round at its size (FP64 b=70 a=40, N and C: relative errors
+                    // 1.23e-16 and 1.44e-16 so, 0.79e-16 and 0.87e-16 here, for 1 % of the
+                    // time at b=64..512)
+                    const T xd = o < cnt ? xs[(f + o) * NR + c] : T(0);
+                    mults_half<T, NR>(v, la, xs, K, tr ? f + o + 1 : 0, tr ? K : f + o);
                     lane_sums<T, NR, 16>(v);
+                    v[0] = fma(ld, xd, v[0]);
                     if (o < cnt) {
                         if (!mute) send_all(y + (f + o) * NR + c, by + p, v[0]);
                         if (h % LC == 0 && c < nr) a.B[(cur.row0 + K0 + f + o) * a.ldb + c0 + c] = v[0];

@@ -1,5 +1,6 @@
-"""GPU: roundings of the small-block sweeps: a solve's quotients round once, and the
-dominant term of a selected inverse's diagonal is added last."""
+"""GPU: roundings of the one-launch sweeps: a small-block solve's quotients round once,
+and the dominant term of a selected inverse's diagonal or of a solve's row is added
+last."""
 
 import numpy as np
 import pytest
@@ -76,3 +77,37 @@ def test_smaller_terms_are_summed_before_the_dominant_one(case, dt):
         ref[1:, :1] = -(2.0 ** -k)
         np.testing.assert_array_equal(np.tril(x, -1), np.tril(ref, -1))
         np.testing.assert_array_equal(np.diag(x)[1:], np.ones(max(m - 1, 0), dt))
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("case", [(2, 5, 4, 1, np.float64), (2, 17, 33, 1, np.float64), (3, 40, 0, 3, np.float64),
+                                  (2, 64, 20, 16, np.float64), (1, 100, 128, 2, np.float64), (3, 128, 1, 5, np.float64),
+                                  (2, 33, 9, 1, np.float32), (2, 90, 0, 4, np.float32), (2, 127, 100, 20, np.float32)])
+def test_a_row_of_a_solve_adds_its_diagonals_term_last(case, trans):
+    """Unit factors with -2**-k in the last row (the first column for L^T), right-hand
+    sides of 2**-k with 1 in that row: it becomes 1 + (rows - 1) 2**-2k.  All terms and
+    their sums below 1 are exact."""
+    n, b, a, nrhs, dt = case
+    k = 27 if dt == np.float64 else 13
+
+    def factor(m):
+        L = np.eye(m, dtype=dt)
+        if m > 1 and trans == "N":
+            L[-1, :-1] = -(2.0 ** -k)
+        elif m > 1:
+            L[1:, 0] = -(2.0 ** -k)
+        return L
+
+    def rows(m, one):
+        x = np.full(m, 2.0 ** -k, dtype=dt)
+        if m:
+            x[-1 if trans == "N" else 0] = one(m)
+        return x
+
+    L = [np.tile(factor(b), (n, 1, 1)), np.zeros((n - 1, b, b), dt), np.zeros((n, a, b), dt), factor(a)]
+    L = [torch.from_numpy(x).cuda() for x in L]
+    B, ref = (np.concatenate([rows(b, one)] * n + [rows(a, one)])[:, None].repeat(nrhs, 1)
+              for one in (lambda m: 1.0, lambda m: dt(1 + (m - 1) * np.longdouble(2) ** (-2 * k))))
+    X = torch.from_numpy(B.copy()).cuda()
+    sg.pobtas(*L, X, trans=trans)
+    np.testing.assert_array_equal(X.cpu().numpy(), ref)
